@@ -271,7 +271,7 @@ PHX_API int phx_traversal_bvh_build(const phx_triangle *tris, uint32_t n, uint32
         CK(cudaMemcpy(d_rank, ranks.data(), 4 * (size_t)n, cudaMemcpyHostToDevice));
         const auto t0 = std::chrono::steady_clock::now();
         std::string msg;
-        const int rc = bvh_device_build(d_tris, n, max_leaf, wide != 0, st, c.db, msg);
+        const int rc = bvh_device_build(d_tris, n, max_leaf, wide != 0, 0.0f, st, c.db, msg);
         if (rc)
             return fail(rc == 2 ? PHX_E_OOM : rc == 1 ? PHX_E_INVALID : PHX_E_CUDA, msg);
         if (bvh_device_finish(d_tris, d_rank, n, c.db, d_rec, d_nrm, d_tan, d_uv, st))

@@ -2,6 +2,7 @@
 // (Renderer::run, src/renderer/renderer.cpp:59-161, with its two host syncs per round) and the
 // graph form (one captured round replayed with no host sync).
 #include "engine.hpp"
+#include "bvh_margin.hpp"
 
 #include <algorithm>
 #include <cmath>
@@ -151,6 +152,39 @@ static float ms_since(std::chrono::steady_clock::time_point t0) {
     return std::chrono::duration<float, std::milli>(std::chrono::steady_clock::now() - t0).count();
 }
 
+// Largest |coordinate| of anything a ray starts from that does not change after set-up: the triangles
+// (`reach` so far), the emissive triangles and the camera.
+static float largest(const phx_f4 &p, float m) {
+    return std::max(m, std::max(std::fabs(p.x), std::max(std::fabs(p.y), std::fabs(p.z))));
+}
+static float geometry_reach(const phx_scene &s, float reach) {
+    for (uint32_t k = 0; k < s.n_emissive_triangles; k++) {
+        const phx_triangle &t = s.emissive_triangles[k];
+        reach = largest(t.v2, largest(t.v1, largest(t.v0, reach)));
+    }
+    const float disk = 2.0f * largest(s.camera.defocus_disk_v, largest(s.camera.defocus_disk_u, 0.0f));
+    return std::max(reach, largest(s.camera.position, 0.0f) + disk);
+}
+
+// The same with the lights: a directional light's photons start from a disk of the scene sphere's
+// radius (at most sqrt(3) * reach, plus the reference box's margin) two radii off its centre, along
+// axes of any length; its direction is not normalised either, which scales the triangle test's errors.
+float ray_reach(float geom, const phx_light *l, uint32_t n) {
+    float m = geom;
+    auto norm = [](const phx_f4 &v) { return std::sqrt(v.x * v.x + v.y * v.y + v.z * v.z); };
+    for (uint32_t k = 0; k < n; k++) {
+        if (l[k].kind == PHX_LIGHT_POINT || l[k].kind == PHX_LIGHT_SPOT)
+            m = std::max(m, norm(l[k].position));
+        else if (l[k].kind == PHX_LIGHT_DIRECTIONAL) {
+            const float d = norm(l[k].direction), r = 1.75f * geom + 0.01f;
+            m = std::max(m, std::max(1.0f, d) * (geom + r * (2.0f * d + norm(l[k].tangent) + norm(l[k].bitangent))));
+        }
+        if (std::isnan(m))
+            break;
+    }
+    return m;
+}
+
 // The SAH traversal tree built on the device (k_bvh.cu) while a host thread builds the reference
 // tree, whose leaf ranks only the last step needs.  done = false: the caller builds on the host
 // (force_ref: the SAH tree is too deep for the traversal stack, use the reference tree).
@@ -171,8 +205,8 @@ static int device_traversal(SceneSlot &S, const phx_scene &s, const phx_params &
     DeviceBvh db;
     std::string msg;
     const bool want_wide = !(p.flags & PHX_F_BINARY_BVH);
-    const int rc =
-        bvh_device_build(tris.as<phx_triangle>(), n, p.bvh_leaf_size ? p.bvh_leaf_size : 4u, want_wide, st, db, msg);
+    const int rc = bvh_device_build(tris.as<phx_triangle>(), n, p.bvh_leaf_size ? p.bvh_leaf_size : 4u, want_wide,
+                                    tight_margin_unit(S.box_reach), st, db, msg);
     ref.join();
     ref_built = ref_ok;
     struct Release {
@@ -220,9 +254,13 @@ int Engine::upload_scene(uint32_t i, const phx_scene &s, const phx_params &p, ui
         return fail(PHX_E_INVALID, "scene has no triangles");
     if (!s.materials || s.n_materials == 0)
         return fail(PHX_E_INVALID, "scene has no materials");
-    for (uint32_t t = 0; t < s.n_triangles; t++)
-        if (s.triangles[t].mat_index >= s.n_materials)
+    float reach = 0.0f;
+    for (uint32_t t = 0; t < s.n_triangles; t++) {
+        const phx_triangle &tr = s.triangles[t];
+        if (tr.mat_index >= s.n_materials)
             return fail(PHX_E_INVALID, "triangle material index out of range");
+        reach = largest(tr.v2, largest(tr.v1, largest(tr.v0, reach)));
+    }
     for (uint32_t l = 0; l < s.n_lights; l++)
         if (s.lights[l].kind == PHX_LIGHT_TEXTURED) {
             uint32_t a, b;
@@ -257,6 +295,9 @@ int Engine::upload_scene(uint32_t i, const phx_scene &s, const phx_params &p, ui
     int r;
     int32_t trav_root = 0;
     bool wide = false, trav_done = false, ref_built = false, force_ref = false;
+    // the 8-bit nodes keep the reference's margin: their planes are rounded once more
+    S.geom_reach = geometry_reach(s, reach);
+    S.box_reach = (p.flags & PHX_F_QUANT_BVH) ? 0.0f : ray_reach(S.geom_reach, s.lights, s.n_lights);
     if (!(p.flags & PHX_F_HOST_BVH) && !(p.flags & PHX_F_REFERENCE_BVH) &&
         (r = device_traversal(S, s, p, st, ref_built, trav_done, force_ref, trav_root, wide)))
         return r;
@@ -271,11 +312,14 @@ int Engine::upload_scene(uint32_t i, const phx_scene &s, const phx_params &p, ui
         bool sah = !(p.flags & PHX_F_REFERENCE_BVH) && !force_ref;
         if (sah) {
             std::vector<uint32_t> ranks = reference_leaf_ranks(S.nodes, s.n_triangles);
-            sah = bvh_build_sah(s.triangles, s.n_triangles, ranks, p.bvh_leaf_size ? p.bvh_leaf_size : 4u, pk) &&
+            sah = bvh_build_sah(s.triangles, s.n_triangles, ranks, p.bvh_leaf_size ? p.bvh_leaf_size : 4u, pk,
+                                tight_margin_unit(S.box_reach)) &&
                   pk.depth + 2 < (uint32_t)TRAV_STACK;
         }
-        if (!sah)
+        if (!sah) {
             bvh_pack(S.nodes, s.triangles, pk);
+            S.box_reach = 0.0f;
+        }
         // 4-wide nodes over the SAH tree (half the dependent node fetches per ray) unless asked for
         // the binary form or the worst-case stack (3 pushes per level) could exceed the traversal stack
         if (sah && !(p.flags & PHX_F_BINARY_BVH)) {

@@ -36,6 +36,8 @@ struct SceneSlot {
     uint32_t trav_depth = 0, trav_inner = 0; // the device traversal tree
     float setup_ms = 0.0f, bvh_ms = 0.0f;     // wall time of the scene setup, of which the trees
     uint32_t n_tris = 0;
+    float geom_reach = 0.0f;  // largest |coordinate| of the triangles, camera and emissive triangles
+    float box_reach = 0.0f;   // bound on every ray origin that the tree's boxes are made for (0: any)
     std::vector<DevBuf> bufs;
     SceneDesc desc{};
     uint64_t total_emitted = 0;
@@ -93,6 +95,7 @@ struct RoundSet {
     u32 *perm = nullptr; // the photon sort's permutation (set by the hash stage)
 };
 
+float ray_reach(float geom, const phx_light *l, uint32_t n);
 uint32_t light_sample_draws(const phx_light *l, uint32_t n, float total_lum);
 
 class Engine {

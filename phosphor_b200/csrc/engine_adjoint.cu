@@ -77,6 +77,13 @@ int Engine::set_lights(const phx_light *l, uint32_t n) {
     CK(cudaMemcpy(S.bufs[13].p, l, sizeof(phx_light) * n, cudaMemcpyHostToDevice));
     CK(cudaMemcpy(S.bufs[14].p, lum.data(), 4 * (size_t)n, cudaMemcpyHostToDevice));
     S.lights.assign(l, l + n);
+    // the tree's boxes are made for rays starting within box_reach: a light moved farther away than any
+    // at set-up gets the reference's margin back (lights that only change power never do)
+    if (S.box_reach > 0.0f && !(ray_reach(S.geom_reach, l, n) <= S.box_reach)) {
+        CK(bvh_device_loosen(S.bufs[0].as<float>(), S.trav_inner, S.desc.wide != 0, st));
+        CK(cudaStreamSynchronize(st));
+        S.box_reach = 0.0f;
+    }
     S.desc.total_lum = lum[n - 1]; // shading.cpp:26
     S.desc.light_draws = light_sample_draws(l, n, S.desc.total_lum);
     invalidate_graph(); // the captured shadow stage depends on the draw count

@@ -1,5 +1,6 @@
 // host.cpp — BVH construction and packing, photon-grid box and scene sphere.
 #include "host.hpp"
+#include "bvh_margin.hpp"
 #include "bvh_quant.hpp"
 
 #include <algorithm>
@@ -12,7 +13,6 @@ namespace phx {
 
 namespace {
 
-constexpr float BBOX_EPS = 1e-3f;
 constexpr float INF = 1e9f;
 constexpr float MIN_CELL_SIZE = 0.001f;
 constexpr float PI = 3.141592654f;
@@ -32,8 +32,9 @@ struct Box {
     float lo[3], hi[3];
 };
 
-// get_bounding_box (bounding_box.h:48-61)
-bool triangle_box(const phx_triangle &t, Box &b) {
+// get_bounding_box (bounding_box.h:48-61); unit > 0: with the traversal tree's own margin
+// (bvh_margin.hpp) in place of the reference's, for the triangles that the reference accepts
+bool triangle_box(const phx_triangle &t, Box &b, float unit = 0.0f) {
     for (int i = 0; i < 3; i++) {
         b.lo[i] = INF;
         b.hi[i] = -INF;
@@ -49,13 +50,14 @@ bool triangle_box(const phx_triangle &t, Box &b) {
     for (int i = 0; i < 3; i++)
         if (b.lo[i] >= INF || b.lo[i] <= -INF || b.hi[i] >= INF || b.hi[i] <= -INF)
             return false;
+    const float c[3][3] = {{t.v0.x, t.v0.y, t.v0.z}, {t.v1.x, t.v1.y, t.v1.z}, {t.v2.x, t.v2.y, t.v2.z}};
+    const float m = box_margin(c, unit);
     for (int i = 0; i < 3; i++) {
-        b.lo[i] -= BBOX_EPS;
-        b.hi[i] += BBOX_EPS;
-    }
-    for (int i = 0; i < 3; i++)
-        if (b.lo[i] == b.hi[i])
+        if (b.lo[i] - BBOX_EPS == b.hi[i] + BBOX_EPS)
             return false;
+        b.lo[i] -= m;
+        b.hi[i] += m;
+    }
     return true;
 }
 
@@ -227,7 +229,7 @@ void bvh_pack(const std::vector<phx_bvh_node> &nodes, const phx_triangle *tris, 
 // Binned SAH (surface area heuristic, MacDonald & Booth 1990; binning after Wald 2007): 32 bins
 // per axis over the primitive centroids, cost = 1 + (A_l N_l + A_r N_r) / A, leaf cost = N.
 bool bvh_build_sah(const phx_triangle *tris, uint32_t n, const std::vector<uint32_t> &ref_rank, uint32_t max_leaf,
-                   PackedBvh &out) {
+                   PackedBvh &out, float unit) {
     if (!tris || n == 0 || n >= (1u << LEAF_FIRST_BITS))
         return false;
     max_leaf = std::max(1u, std::min(max_leaf, 16u));
@@ -238,7 +240,7 @@ bool bvh_build_sah(const phx_triangle *tris, uint32_t n, const std::vector<uint3
     std::vector<Prim> P(n);
     for (uint32_t i = 0; i < n; i++) {
         Box b;
-        if (!triangle_box(tris[i], b))
+        if (!triangle_box(tris[i], b, unit))
             return false;
         for (int a = 0; a < 3; a++) {
             P[i].lo[a] = b.lo[a];

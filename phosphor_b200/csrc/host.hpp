@@ -32,9 +32,10 @@ std::vector<uint32_t> reference_leaf_ranks(const std::vector<phx_bvh_node> &node
 // The reference tree itself re-packed as child pairs (one triangle per leaf).
 void bvh_pack(const std::vector<phx_bvh_node> &nodes, const phx_triangle *tris, PackedBvh &out);
 // A binned-SAH tree over the same expanded triangle boxes (bounding_box.h:48-61), leaves of up to
-// max_leaf triangles; triangle records carry the reference leaf rank for tie-breaking.
+// max_leaf triangles; triangle records carry the reference leaf rank for tie-breaking.  unit > 0: the
+// boxes reach past their triangles by box_margin(unit) (bvh_margin.hpp) instead of the reference's 1e-3.
 bool bvh_build_sah(const phx_triangle *tris, uint32_t n, const std::vector<uint32_t> &ref_rank, uint32_t max_leaf,
-                   PackedBvh &out);
+                   PackedBvh &out, float unit = 0.0f);
 
 // Collapses the child-pair tree into 4-wide nodes (each node pulls up the grandchildren of its
 // largest inner children until it has 4): 7 float4 per node, SoA {minx[4], maxx[4], miny[4],

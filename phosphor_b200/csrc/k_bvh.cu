@@ -28,6 +28,7 @@
 #include <cstring>
 #include <vector>
 
+#include "bvh_margin.hpp"
 #include "bvh_quant.hpp"
 #include "kernels.hpp"
 
@@ -42,7 +43,6 @@ constexpr int NB_SMALL = 32;       // and below
 constexpr u32 NB_SWITCH = 256;
 constexpr u32 NO_PARENT = 0xFFFFFFFFu;
 constexpr u32 MAX_LEVELS = 1u << 16;
-constexpr float BBOX_EPS = 1e-3f;  // bounding_box.h expansion
 constexpr float BOX_INF = 1e9f;    // bounding_box.h "infinite" coordinate
 constexpr float BIG = 1e30f;       // the host builder's empty-box bounds
 
@@ -663,8 +663,8 @@ __global__ void __launch_bounds__(256) k_big_scatter(const Chunk *chunks, const 
 
 // ---- primitives, numbering, records ---------------------------------------------------------
 
-// get_bounding_box (bounding_box.h:48-61) of every triangle, expanded by BBOX_EPS
-__global__ void k_prims(const phx_triangle *tris, u32 n, Prim *out, u32 *err) {
+// get_bounding_box (bounding_box.h:48-61) of every triangle, expanded by its margin (bvh_margin.hpp)
+__global__ void k_prims(const phx_triangle *tris, u32 n, float unit, Prim *out, u32 *err) {
     const u32 i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n)
         return;
@@ -681,15 +681,29 @@ __global__ void k_prims(const phx_triangle *tris, u32 n, Prim *out, u32 *err) {
         }
         bad |= lo[a] >= BOX_INF || lo[a] <= -BOX_INF || hi[a] >= BOX_INF || hi[a] <= -BOX_INF;
     }
+    const float m = box_margin(v, unit);
     for (int a = 0; a < 3; a++) {
-        lo[a] = __fsub_rn(lo[a], BBOX_EPS);
-        hi[a] = __fadd_rn(hi[a], BBOX_EPS);
-        bad |= lo[a] == hi[a];
+        bad |= __fsub_rn(lo[a], BBOX_EPS) == __fadd_rn(hi[a], BBOX_EPS);
+        lo[a] = __fsub_rn(lo[a], m);
+        hi[a] = __fadd_rn(hi[a], m);
     }
     if (bad)
         atomicOr(err, ERR_DEGENERATE);
     out[i].lo = make_float4(lo[0], lo[1], lo[2], __uint_as_float(i));
     out[i].hi = make_float4(hi[0], hi[1], hi[2], 0.0f);
+}
+
+// Every box of a tree's nodes (child pairs or 4-wide) widened to hold the reference's margin.  An empty
+// slot's box (1e30, -1e30) stays as it is: 1e-3 vanishes beside 1e30.
+__global__ void k_loosen(float *nodes, u32 n_nodes, bool wide) {
+    const u32 i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n_nodes)
+        return;
+    float *o = nodes + (size_t)i * (wide ? 28 : 16);
+    for (int k = 0; k < (wide ? 24 : 12); k++) {
+        const bool lower = wide ? ((k >> 2) & 1) == 0 : (k & 1) == 0; // rows min, max or pairs (min, max)
+        o[k] = lower ? __fsub_rn(o[k], BBOX_EPS) : __fadd_rn(o[k], BBOX_EPS);
+    }
 }
 
 // inner nodes under each node of one level (children are deeper, already counted)
@@ -984,8 +998,14 @@ void DeviceBvh::release() {
     leaves = nullptr;
 }
 
-int bvh_device_build(const phx_triangle *tris, u32 n, u32 max_leaf, bool widen, cudaStream_t st, DeviceBvh &out,
-                     std::string &err) {
+cudaError_t bvh_device_loosen(float *nodes, u32 n_nodes, bool wide, cudaStream_t st) {
+    if (n_nodes)
+        k_loosen<<<blocks_for(n_nodes, 256), 256, 0, st>>>(nodes, n_nodes, wide);
+    return cudaGetLastError();
+}
+
+int bvh_device_build(const phx_triangle *tris, u32 n, u32 max_leaf, bool widen, float unit, cudaStream_t st,
+                     DeviceBvh &out, std::string &err) {
     out.release();
     out = DeviceBvh{};
     if (!tris || n == 0 || n >= (1u << LEAF_FIRST_BITS)) {
@@ -1038,7 +1058,7 @@ int bvh_device_build(const phx_triangle *tris, u32 n, u32 max_leaf, bool widen, 
     cudaMemsetAsync(rec, 0, (size_t)n * 16 * 4, st);
     cudaMemsetAsync(out.leaf_tri, 0, (size_t)n * 4, st);
     cudaMemsetAsync(ctr, 0, sizeof(Counters), st);
-    k_prims<<<blocks_for(n, 256), 256, 0, st>>>(tris, n, pa, &ctr->err);
+    k_prims<<<blocks_for(n, 256), 256, 0, st>>>(tris, n, unit, pa, &ctr->err);
     {
         BuildArgs A{};
         A.ctr = ctr;

@@ -130,8 +130,11 @@ struct DeviceBvh {
     int wroot = 0;
     void release();
 };
-int bvh_device_build(const phx_triangle *tris, u32 n, u32 max_leaf, bool widen, cudaStream_t st, DeviceBvh &out,
-                     std::string &err);
+// unit: 0 for the reference's box margin, else the tight one's (bvh_margin.hpp)
+int bvh_device_build(const phx_triangle *tris, u32 n, u32 max_leaf, bool widen, float unit, cudaStream_t st,
+                     DeviceBvh &out, std::string &err);
+// Widens every box of uploaded nodes (child pairs, or 4-wide) by the reference's margin
+cudaError_t bvh_device_loosen(float *nodes, u32 n_nodes, bool wide, cudaStream_t st);
 // 4-wide nodes -> 8-bit child boxes (bvh_quant.hpp), one thread per node
 cudaError_t bvh_device_quantize(const float *wnodes, u32 n, u32 *out, cudaStream_t st);
 int bvh_device_finish(const phx_triangle *tris, const u32 *rank, u32 n, DeviceBvh &b, float4 *trirec, float4 *nrm,

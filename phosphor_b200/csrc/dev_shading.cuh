@@ -304,9 +304,9 @@ struct BsdfSample {
     u32 event;
 };
 
-// shading.h:150-213
-PHX_SHADE_BSDF BsdfSample sample_bsdf(Rng *rng, const ShadingContext &ctx, float4 sn, float4 gn, float4 view, IorStack *ior,
-                              bool front) {
+// shading.h:150-213; *half_out receives the microfacet normal
+PHX_DI BsdfSample sample_bsdf_h(Rng *rng, const ShadingContext &ctx, float4 sn, float4 gn, float4 view, IorStack *ior,
+                                bool front, float4 *half_out) {
     BsdfSample s;
     // one frame of the shading normal serves the microfacet sample and a diffuse direction
     float4 tn, bn;
@@ -314,6 +314,7 @@ PHX_SHADE_BSDF BsdfSample sample_bsdf(Rng *rng, const ShadingContext &ctx, float
     float4 hr;
     bool has_hr;
     float4 h = ggx_sample_vndf_tbn(rng, sn, tn, bn, gn, view, ctx.roughness, &hr, &has_hr);
+    *half_out = h;
     // safe_reflect(-view, h, gn), reusing reflect(-view, h) from the microfacet sample
     auto reflect_h = [&]() {
         float4 r = has_hr ? hr : reflect(-view, h);
@@ -372,6 +373,12 @@ PHX_SHADE_BSDF BsdfSample sample_bsdf(Rng *rng, const ShadingContext &ctx, float
     s.throughput = ctx.base_color;
     s.event = BSDF_DIFFUSE;
     return s;
+}
+
+PHX_SHADE_BSDF BsdfSample sample_bsdf(Rng *rng, const ShadingContext &ctx, float4 sn, float4 gn, float4 view, IorStack *ior,
+                              bool front) {
+    float4 h;
+    return sample_bsdf_h(rng, ctx, sn, gn, view, ior, front, &h);
 }
 
 // ---- light_sampling.h:18-390 -------------------------------------------------------------------
@@ -581,6 +588,13 @@ PHX_DI bool light_fragment(Rng *rng, const SceneDesc &sc, float4 pos, float4 nor
 }
 PHX_SHADE_NEE bool sample_light_fragment(Rng *rng, const SceneDesc &sc, float4 pos, float4 normal, LightFragment *out) {
     return light_fragment(rng, sc, pos, normal, out);
+}
+
+// Whether a scene's specular NEE samples are drawn by the shadow kernel (each thread its own
+// sample, from the event's RNG state advanced past the samples before it): possible when every
+// light sample takes the same number of draws; the event record needs four sample slots.
+PHX_DI bool spec_drawn_in_shadow(const SceneDesc &sc) {
+    return sc.light_draws != LIGHT_DRAWS_VARY && sc.direct_samples >= 4;
 }
 
 // light_sampling.h:302-333

@@ -675,12 +675,9 @@ void Engine::enq_seeds_r(RoundSet &R, cudaStream_t s) {
     ev(ST_SEEDS, true, s);
 }
 
-void Engine::enq_trace_r(RoundSet &R, cudaStream_t s) {
-    ev(ST_TRACE, false, s);
+TraceOut Engine::trace_out(const RoundSet &R) const {
     TraceOut o{R.hp[0], R.hp[1], R.hp[2], R.hp[3], R.hp[4], R.hp[5], R.nee_ray, R.nee_val, R.stash_sn, R.stash_rng};
-    const LaunchCtx l = lc(R);
-    const bool spec = spec_deferred();
-    if (spec) {
+    if (spec_deferred()) {
         o.spec_ray = R.spec_ray;
         o.spec_val = R.spec_val;
         o.spec_org = R.spec_org;
@@ -691,8 +688,25 @@ void Engine::enq_trace_r(RoundSet &R, cudaStream_t s) {
         o.def_prefix = R.def_prefix;
         o.def_val = R.def_val;
         o.def_tag = R.def_tag;
-        cudaMemsetAsync(R.spec_next, 0, sizeof(u32), s);
     }
+    return o;
+}
+
+// Every sample of a hit point is one ray when the only light is a point, spot or directional one.
+bool Engine::one_sample() const {
+    return sc.size() == 1 && shard.world == 1 && sc[0].lights.size() == 1 &&
+           sc[0].lights[0].kind != PHX_LIGHT_TEXTURED;
+}
+
+void Engine::enq_trace_r(RoundSet &R, cudaStream_t s) {
+    ev(ST_TRACE, false, s);
+    if (!in_adjoint)
+        adj_live = ADJ_NO_ROUND;
+    const TraceOut o = trace_out(R);
+    const LaunchCtx l = lc(R);
+    const bool spec = spec_deferred();
+    if (spec)
+        cudaMemsetAsync(R.spec_next, 0, sizeof(u32), s);
     launch_trace(l, o, (int)tune.trace_block, (int)tune.persistent, (int)tune.trace_blocks_per_sm, R.queue,
                  untextured(), s);
     ev(ST_TRACE, true, s);
@@ -702,11 +716,8 @@ void Engine::enq_trace_r(RoundSet &R, cudaStream_t s) {
         transmissive = transmissive || sl.desc.any_transmissive != 0;
         presample = presample || sl.desc.light_draws == LIGHT_DRAWS_VARY;
     }
-    // every sample of a hit point is one ray when the only light is a point, spot or directional one
-    const bool per_pixel = sc.size() == 1 && shard.world == 1 && sc[0].lights.size() == 1 &&
-                           sc[0].lights[0].kind != PHX_LIGHT_TEXTURED;
     const int kind = !transmissive ? SHADOW_OPAQUE : untextured() ? SHADOW_CLEAR : SHADOW_GENERAL;
-    launch_shadow(l, o, kind, presample, per_pixel, sc[0].desc.n_pixels,
+    launch_shadow(l, o, kind, presample, one_sample(), sc[0].desc.n_pixels,
                   sc.size() == 1 ? &sc[0].desc : nullptr, s);
     launch_nee_resolve(l, o, s);
     if (spec)
@@ -717,7 +728,9 @@ void Engine::enq_trace_r(RoundSet &R, cudaStream_t s) {
 
 void Engine::enq_emit_r(RoundSet &R, cudaStream_t s) {
     ev(ST_EMIT, false, s);
-    EmitOut o{R.slot_pos, R.slot_pd, R.counts};
+    if (!in_adjoint)
+        adj_live = ADJ_NO_ROUND;
+    EmitOut o{R.slot_pos, R.slot_pd, R.counts, in_adjoint ? adj_slot_pow.as<float4>() : nullptr};
     launch_emit(lc(R), o, (int)tune.emit_block, (int)tune.persistent, (int)tune.emit_blocks_per_sm, R.queue + 1,
                 untextured(), photon_prestart(), s);
     ev(ST_EMIT, true, s);
@@ -730,6 +743,8 @@ void Engine::enq_emit_r(RoundSet &R, cudaStream_t s) {
 
 void Engine::enq_hash_sort_r(RoundSet &R, cudaStream_t s) {
     ev(ST_HASH, false, s);
+    if (!in_adjoint)
+        adj_live = ADJ_NO_ROUND;
     cudaMemsetAsync(R.cell_count, 0, 4 * ((size_t)total_cells + 1), s);
     launch_hash(lc(R), gb(R), R.ntotal, max_photons, s);
     ev(ST_HASH, true, s);
@@ -790,6 +805,7 @@ void Engine::accumulate_profile() {
 void Engine::invalidate_graph() {
     if (st)
         cudaStreamSynchronize(st);
+    adj_live = ADJ_NO_ROUND; // a tuning, material or light change: what the buffers hold may be of another form
     if (gexec)
         cudaGraphExecDestroy(gexec);
     if (graph)

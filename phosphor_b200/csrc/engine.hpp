@@ -146,6 +146,7 @@ class Engine {
     int shard_round();
     bool any_active() const;
     bool untextured() const; // no material of any scene has a texture (indices are fixed at set-up)
+    bool one_sample() const; // a hit point's NEE samples are all the same ray
     bool photon_prestart() const; // every scene keeps >= 3 photon slots per path (k_emit_start)
 
     // differentiation (single-scene engines; engine_adjoint.cu)
@@ -173,6 +174,7 @@ class Engine {
     GridBufs gb() const { return gb(rs0); }
     LaunchCtx lc(const RoundSet &R) const;
     GridBufs gb(const RoundSet &R) const;
+    TraceOut trace_out(const RoundSet &R) const;
     void enq_seeds_r(RoundSet &R, cudaStream_t s);
     void enq_trace_r(RoundSet &R, cudaStream_t s);
     void enq_emit_r(RoundSet &R, cudaStream_t s);
@@ -223,6 +225,8 @@ class Engine {
         adj_grad;
     uint32_t adj_rounds = 0;
     bool adj_ready = false, adj_k_ready = false, in_adjoint = false;
+    static constexpr uint32_t ADJ_NO_ROUND = 0xffffffffu;
+    uint32_t adj_live = ADJ_NO_ROUND; // recorded round whose hit points, samples and photons the buffers hold
     float *rec_r2 = nullptr, *rec_ratio = nullptr; // recording targets of the gather (forward pass)
 
     // pixel order of the gather (pixels grouped by photon-grid cell)

@@ -159,8 +159,8 @@ __global__ void __launch_bounds__(128) k_emit_start(LaunchCtx lc, EmitOut out) {
 
 // Consumes the pending query; returns true while the path continues.  NOTEX: no material of the
 // context has a texture (texture indices never change after set-up), so every texture branch is
-// compiled out of this instance.
-template <bool NOTEX>
+// compiled out of this instance.  POW: the stored photons' unquantised power is kept too (out.slot_pow).
+template <bool NOTEX, bool POW>
 PHX_DI bool pp_advance(PhotonPath &p, bool hit, const Hit &h, const EmitOut &out) {
     const SceneDesc &sc = *p.sc;
     if (!hit)
@@ -202,6 +202,8 @@ PHX_DI bool pp_advance(PhotonPath &p, bool hit, const Hit &h, const EmitOut &out
     if (bs.event == BSDF_DIFFUSE && dot(p.dir, sh.normal) < 0.0f) {
         out.slot_pos[p.slot] = sh.position;
         out.slot_pd[p.slot] = make_uint2(encode_rgbe(p.power), encode_oct(p.dir));
+        if constexpr (POW)
+            out.slot_pow[p.slot] = p.power;
         p.slot += sc.n_emit;
         p.n_out++;
     }
@@ -214,7 +216,7 @@ PHX_DI bool pp_advance(PhotonPath &p, bool hit, const Hit &h, const EmitOut &out
     return p.depth < sc.max_bounces;
 }
 
-template <bool NOTEX, bool PRE>
+template <bool NOTEX, bool PRE, bool POW = false>
 __global__ void __launch_bounds__(128, PHX_EMIT_MINB) k_emit_persistent(LaunchCtx lc, EmitOut out, u32 *queue) {
     const u32 lane = threadIdx.x & 31u;
     const u32 lt_mask = (1u << lane) - 1u;
@@ -250,7 +252,7 @@ __global__ void __launch_bounds__(128, PHX_EMIT_MINB) k_emit_persistent(LaunchCt
         if (active) {
             Hit h;
             const bool hit = intersect(*p.sc, p.origin, p.dir, EPS, INF, &h, &ovf);
-            if (!pp_advance<NOTEX>(p, hit, h, out)) {
+            if (!pp_advance<NOTEX, POW>(p, hit, h, out)) {
                 out.counts[p.gid] = p.n_out;
                 active = false;
             }
@@ -264,11 +266,20 @@ void launch_emit(const LaunchCtx &lc, const EmitOut &out, int block, int persist
                  bool untextured, bool prestart, cudaStream_t st) {
     if (lc.emit_hi <= lc.emit_lo)
         return;
-    if (persistent && queue && !out.slot_pow) {
+    if (persistent && queue) {
         cudaMemsetAsync(queue, 0, sizeof(u32), st);
         if (prestart)
             k_emit_start<<<(lc.emit_hi - lc.emit_lo + 127) / 128, 128, 0, st>>>(lc, out);
         int grid = g_sm_count * (blocks_per_sm > 0 ? blocks_per_sm : 8);
+        if (out.slot_pow) { // the adjoint's rounds
+            if (untextured && prestart)
+                k_emit_persistent<true, true, true><<<grid, 128, 0, st>>>(lc, out, queue);
+            else if (prestart)
+                k_emit_persistent<false, true, true><<<grid, 128, 0, st>>>(lc, out, queue);
+            else
+                k_emit_persistent<false, false, true><<<grid, 128, 0, st>>>(lc, out, queue);
+            return;
+        }
         // untextured: emit 4.52 -> 4.44 ms (caustic), 2.82 -> 2.73 ms (atrium)
         if (untextured && prestart)
             k_emit_persistent<true, true><<<grid, 128, 0, st>>>(lc, out, queue);

@@ -261,13 +261,6 @@ PHX_DI void cp_start(CameraPath &p, const SceneDesc *sc, u32 seed, u32 tid, u32 
     p.t_max = INF;
 }
 
-// Whether a scene's specular NEE samples are drawn by the shadow kernel (each thread its own
-// sample, from the event's RNG state advanced past the samples before it): possible when every
-// light sample takes the same number of draws; the event record needs four sample slots.
-PHX_DI bool spec_drawn_in_shadow(const SceneDesc &sc) {
-    return sc.light_draws != LIGHT_DRAWS_VARY && sc.direct_samples >= 4;
-}
-
 // One sample of direct_lighting_specular (light_sampling.h:355-390) up to its shadow query: false
 // when it contributes nothing (no RNG draw depends on a shadow query's outcome), else the light
 // fragment and the weight m of its transmittance.

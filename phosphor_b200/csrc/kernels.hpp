@@ -78,7 +78,7 @@ struct EmitOut {
     float4 *slot_pos;
     uint2 *slot_pd;    // (rgbe power, octahedral direction)
     u32 *counts;       // per photon path (global emit index)
-    float4 *slot_pow;  // optional (one-thread-per-path form only): unquantised power per slot
+    float4 *slot_pow;  // optional: unquantised power per slot
 };
 // untextured: no material of the context has a texture.  prestart: every scene has at least three
 // photon slots per path (max_bounces >= 3), so the lane-refill form can draw the paths' light
@@ -185,6 +185,9 @@ struct AdjBufs {
     double *grad;          // 4 per material (base r, g, b, roughness), then 3 per light (power r, g, b)
     u32 n_params, n_mat;
     float inv_rounds;
+    TraceOut tr;           // the round's camera pass with its recorded NEE samples (def_cnt null: not recorded)
+    u32 same_samples;      // direct_samples where a hit point's samples are all one ray, else 0
+    u32 occluders;         // 1: materials transmit, the recorded samples' occluders are looked up
     u32 block_sums;        // 1: per-block partial sums in 4*n_params bytes of shared memory
 };
 void launch_gather_adj(const LaunchCtx &lc, const GatherBufs &g, const AdjBufs &ab, cudaStream_t st);
@@ -192,6 +195,9 @@ void launch_trace_adj(const LaunchCtx &lc, const AdjBufs &ab, cudaStream_t st);
 void launch_emit_adj(const LaunchCtx &lc, const AdjBufs &ab, cudaStream_t st);
 void launch_compact_pow(const LaunchCtx &lc, const float4 *slot_pow, const u32 *counts, const u32 *offsets,
                         float4 *ph_pow, cudaStream_t st);
+// dL/dI from three floats a pixel to float4, and zeroes gphi of the *n stored photons
+void launch_adj_begin(const float *g3, float4 *g4, u32 n_pix, cudaStream_t st);
+void launch_adj_clear(float4 *gphi, const u32 *n, u64 n_max, cudaStream_t st);
 void launch_adj_scale(const float *ratio, float *kscale, const float4 *flux, u32 n_pix, u32 rounds, float inv_n,
                       cudaStream_t st);
 void launch_adj_image(const float4 *flux, const float4 *radiance, u32 n_pix, float inv_rounds, float inv_n, float *img,

@@ -10,172 +10,219 @@
 // not materialised: the cells are contiguous, so end(h) = start(h+1).
 #include "kernels.hpp"
 
-// Photon records loaded ahead per step of a cell's loop (4: gather 2.40 -> 2.30 ms on the caustic
-// workload, 3.93 -> 3.56 ms on the atrium one, against 2).
-#ifndef PHX_GATHER_AHEAD
-#define PHX_GATHER_AHEAD 4
-#endif
-
-// Each cell's photon range loaded while the previous cell's photons are summed (1), or after
-// (0: one more dependent load round trip per searched cell).
-#ifndef PHX_GATHER_NEXT_CELL
-#define PHX_GATHER_NEXT_CELL 1
-#endif
-
 namespace phx {
 
-PHX_DI void gather_pixel(const SceneDesc &sc, u32 gpix, const GatherBufs &g) {
-    float4 ge = g.hp_emission[gpix];
-    float4 rso = g.radiance[gpix];
-    float4 r = f4(ge.x, ge.y, ge.z, 0.0f);
-    if (ge.w == 0.0f) {
-        g.radiance[gpix] = rso + r;
-        if (g.rec_r2) {
-            g.rec_r2[gpix] = 0.0f;
-            g.rec_ratio[gpix] = 1.0f;
-        }
-        return;
-    }
-    float4 direct = g.hp_direct[gpix];
-    r.x += direct.x;
-    r.y += direct.y;
-    r.z += direct.z;
-    g.radiance[gpix] = rso + r;
-    float4 fso = g.flux[gpix];
-    float wso = g.weight[gpix];
-    const GridDev grid = sc.grid;
-    float r_sq = fso.w;
-    if (r_sq < EPS) {
-        float hx = grid.cx * 0.5f, hy = grid.cy * 0.5f, hz = grid.cz * 0.5f;
-        r_sq = hx * hx + hy * hy + hz * hz;
-    }
-    const float4 pos = g.hp_pos[gpix];
-    const float4 nrm = g.hp_normal[gpix];
-    float4 nf = zero4();
-    float found = 0.0f;
-    const u32 *cs = g.cell_start + sc.cell_base;
-    const float denom = 2.0f * r_sq;
-    // hit point in cell units, for the cell-distance test below
-    const float qx = (pos.x - grid.ox) / grid.cx, qy = (pos.y - grid.oy) / grid.cy, qz = (pos.z - grid.oz) / grid.cz;
-    const u32 G = grid.g;
-    // One photon's contribution, in the reference's arithmetic (photon_hash.h:84-101).
-    auto add = [&](const float4 p, u32 k) {
-        const float dx = pos.x - p.x, dy = pos.y - p.y, dz = pos.z - p.z, dw = pos.w - 0.0f;
-        const float dsq = ((dx * dx + dy * dy) + dz * dz) + dw * dw;
-        if (dsq < r_sq) {
-            const float4 pd = __ldg(&g.s_dir[k]); // decode_oct(p.w), decoded once per round
-            if (!(dot(pd, nrm) > 0.0f)) {
-                const float w = GAUSS_ALPHA * (1.0f - (1.0f - pm_expf((-GAUSS_BETA) * dsq / denom)) / GAUSS_DENOM);
-                nf += w * __ldg(&g.s_pow[k]); // decode_rgbe(s_power[k])
-                found += w;
+// x / y from r = 1 / y, for the many x of one y.  Markstein's theorem ("Computation of elementary functions on
+// the IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990): if r is 1/y rounded to nearest and q
+// within one ulp of x/y, then q + (x - q y) r, each step one fused multiply-add, is x/y rounded to
+// nearest.  x r alone is within 1.5 ulp, so a first step brings it within one and the second is exact.
+// Needs x/y, x and x 2^-24 in the normal range.
+PHX_DI float div_known(float x, float y, float r) {
+    float q = x * r;
+    q = __fmaf_rn(__fmaf_rn(-q, y, x), r, q);
+    return __fmaf_rn(__fmaf_rn(-q, y, x), r, q);
+}
+// x / GAUSS_DENOM for x = 0 or in [2^-30, 1.5]: one step is enough (every such x was checked).
+PHX_DI float div_gauss(float x) {
+    constexpr float r = 1.0f / GAUSS_DENOM;
+    const float q = x * r;
+    return __fmaf_rn(__fmaf_rn(-q, GAUSS_DENOM, x), r, q);
+}
+
+// pm_expf for t in [-1, 0]: its operations without its range checks.
+PHX_DI float exp_unit(float t) {
+    const float kf = floorf(t * PM_LOG2E + 0.5f); // 0 or -1
+    float r = t - kf * PM_LN2_HI;
+    r = r - kf * PM_LN2_LO;
+    float p = 1.984126984126984e-04f;
+    p = p * r + 1.388888888888889e-03f;
+    p = p * r + 8.333333333333333e-03f;
+    p = p * r + 4.1666666666666664e-02f;
+    p = p * r + 1.6666666666666666e-01f;
+    p = p * r + 0.5f;
+    p = p * r + 1.0f;
+    p = p * r + 1.0f;
+    return kf < 0.0f ? p * 0.5f : p;
+}
+
+// One pixel per thread, in two alternating phases.  The lanes of a warp walk their cells' photons four at a
+// time and only queue those inside the radius (a few instructions each, no branch to a rare long
+// side); once some lane's queue could not take four more, all lanes work their queues off together,
+// three photons at a time with their loads in flight together.  Adding each photon where it is found
+// instead ran the 60 instructions of a contribution for the one lane in three or four whose photon
+// passes: 10 lanes an instruction, now 17.  A queue keeps the order in which its pixel finds its
+// photons, so each sum is the same.  Measured a round, before and after: 2.25 -> 1.67 ms (caustic
+// workload), 3.88 -> 1.82 (atrium), 0.40 -> 0.25 (512 x 512 Cornell).  16 queue places, 8 blocks per SM
+// and batches of 3 measured best of 12..32, 6..12 and 1..4 (more blocks spill, smaller queues empty
+// while most lanes hold few).
+constexpr u32 GQ_CAP = 16, GQ_AHEAD = 4, GQ_BATCH = 3;
+__global__ void __launch_bounds__(128, 8) k_gather(LaunchCtx lc, GatherBufs g) {
+    __shared__ u32 q_k[GQ_CAP][128];
+    __shared__ float q_d[GQ_CAP][128];
+    constexpr u32 FULL = 0xffffffffu;
+    const u32 tid = threadIdx.x;
+    u32 gpix = blockIdx.x * blockDim.x + tid;
+    bool gathering = false;
+    float4 pos = zero4(), nrm = zero4(), nf = zero4();
+    float r_sq = 0.0f, found = 0.0f;
+    u32 wx = 0, wy = 0, wz = 0, near = 0; // cell coordinates per axis, and the cells within the radius
+    const SceneDesc *scp = lc.scenes;
+    if (gpix < lc.total_pixels) {
+        if (g.order)
+            gpix = __ldg(&g.order[gpix]);
+        scp = lc.scenes + (lc.n_scenes == 1 ? 0 : find_scene(lc.pix_bases, lc.n_scenes, gpix));
+        if (scp->active) {
+            const float4 ge = g.hp_emission[gpix];
+            const float4 rso = g.radiance[gpix];
+            float4 r = f4(ge.x, ge.y, ge.z, 0.0f);
+            if (ge.w == 0.0f) {
+                g.radiance[gpix] = rso + r;
+                if (g.rec_r2) {
+                    g.rec_r2[gpix] = 0.0f;
+                    g.rec_ratio[gpix] = 1.0f;
+                }
+            } else {
+                const float4 direct = g.hp_direct[gpix];
+                r.x += direct.x;
+                r.y += direct.y;
+                r.z += direct.z;
+                g.radiance[gpix] = rso + r;
+                gathering = true;
             }
         }
-    };
-    // The 27 cells in the reference's order (photon_hash.h:65-82), each in sorted (canonical)
-    // photon order.  A cell whose box lies farther than the search radius from the hit point holds
-    // no photon with dsq < r_sq, so it adds nothing and is skipped; the box is widened by 1/1024
-    // of a cell on every side so that rounding in get_hash (which decides a photon's cell) and in
-    // this test can never skip a photon that would count.
-    constexpr float M = 1.0f / 1024.0f;
-    // cell hash of neighbour offset i (0 outside the grid), and whether its box can hold a photon
-    // within the radius
-    // get_hash of a neighbour position works axis by axis, and an axis's coordinate only takes the
-    // three values pos + {-1, 0, 1} * cell: each axis's three cell coordinates are computed once,
-    // with the same operations get_hash applies (0xff: outside the grid, which has at most 255
-    // cells per axis), and packed one byte per offset.
-    const float gf = (float)G;
-    auto axis_cells = [&](float p, float o, float c) -> u32 {
-        u32 w = 0;
+    }
+    const SceneDesc &sc = *scp;
+    const GridDev grid = sc.grid;
+    const u32 *cs = g.cell_start + sc.cell_base;
+    const u32 G = grid.g;
+    if (gathering) {
+        r_sq = g.flux[gpix].w;
+        if (r_sq < EPS) {
+            float hx = grid.cx * 0.5f, hy = grid.cy * 0.5f, hz = grid.cz * 0.5f;
+            r_sq = hx * hx + hy * hy + hz * hz;
+        }
+        pos = g.hp_pos[gpix];
+        nrm = g.hp_normal[gpix];
+        // The 27 cells in the reference's order (photon_hash.h:65-82), each in sorted (canonical)
+        // photon order.  A cell whose box lies farther than the search radius from the hit point holds
+        // no photon with dsq < r_sq, so it adds nothing and is skipped; the box is widened by 1/1024
+        // of a cell on every side so that rounding in get_hash (which decides a photon's cell) and in
+        // this test can never skip a photon that would count.
+        // get_hash of a neighbour position works axis by axis, and an axis's coordinate only takes the
+        // three values pos + {-1, 0, 1} * cell: each axis's three cell coordinates are computed once,
+        // with the same operations get_hash applies, and packed one byte per offset; an axis's three
+        // squared distances decide the cells together (infinite outside the grid, which has at most 255
+        // cells per axis).
+        constexpr float M = 1.0f / 1024.0f;
+        const float gf = (float)G;
+        float d2[3][3];
+        auto axis_cells = [&](float p, float o, float c, float (&d)[3]) -> u32 {
+            const float q0 = (p - o) / c; // the hit point in cell units
+            u32 w = 0;
 #pragma unroll
-        for (int k = 0; k < 3; k++) {
-            float q = p;
-            q += (float)(k - 1) * c;
-            const float f = (q - o) / c;
-            const u32 ci = (f < 0.0f || f >= gf) ? 0xffu : (u32)f;
-            w |= ci << (8 * k);
+            for (int k = 0; k < 3; k++) {
+                float q = p;
+                q += (float)(k - 1) * c;
+                const float f = (q - o) / c;
+                const bool in = !(f < 0.0f || f >= gf);
+                const u32 ci = in ? (u32)f : 0u;
+                const float gap = fmaxf(fmaxf(((float)ci - M) - q0, q0 - ((float)ci + (1.0f + M))), 0.0f) * c;
+                d[k] = in ? gap * gap : __int_as_float(0x7f800000);
+                w |= ci << (8 * k);
+            }
+            return w;
+        };
+        wx = axis_cells(pos.x, grid.ox, grid.cx, d2[0]);
+        wy = axis_cells(pos.y, grid.oy, grid.cy, d2[1]);
+        wz = axis_cells(pos.z, grid.oz, grid.cz, d2[2]);
+#pragma unroll
+        for (u32 c = 0; c < 27; c++) {
+            const float dx = d2[0][c % 3], dy = d2[1][(c / 3) % 3], dz = d2[2][c / 9];
+            if (!((dx + dy) + dz > r_sq) && dx + dy + dz < __int_as_float(0x7f800000))
+                near |= 1u << c;
         }
-        return w;
-    };
-    const u32 wx = axis_cells(pos.x, grid.ox, grid.cx), wy = axis_cells(pos.y, grid.oy, grid.cy),
-              wz = axis_cells(pos.z, grid.oz, grid.cz);
-    auto cell_of = [&](u32 i, bool *near) -> u32 {
-        const u32 hx = (wx >> (8 * (i % 3))) & 0xffu;
-        const u32 hy = (wy >> (8 * ((i / 3) % 3))) & 0xffu;
-        const u32 hz = (wz >> (8 * ((i / 9) % 3))) & 0xffu;
-        if (hx == 0xffu || hy == 0xffu || hz == 0xffu) {
-            *near = false;
-            return 0;
-        }
+    }
+    const float denom = 2.0f * r_sq, dw = pos.w - 0.0f;
+    const float rdenom = 1.0f / denom;
+    const float dsq_min = denom > 1e-18f && denom < 1e18f ? 1e-30f : __int_as_float(0x7f800000);
+    // the photon range of the next cell of `near`
+    auto next_cell = [&](u32 *lo, u32 *hi) {
+        const u32 c = (u32)__ffs(near) - 1u, c3 = c / 3u;
+        near &= near - 1u;
+        const u32 hx = (wx >> (8u * (c - 3u * c3))) & 0xffu, hy = (wy >> (8u * (c3 % 3u))) & 0xffu,
+                  hz = (wz >> (8u * (c / 9u))) & 0xffu;
         const u32 h = G * G * hx + G * hy + hz + 1; // get_hash's cell index
-        const float gx = fmaxf(fmaxf(((float)hx - M) - qx, qx - ((float)hx + (1.0f + M))), 0.0f) * grid.cx;
-        const float gy = fmaxf(fmaxf(((float)hy - M) - qy, qy - ((float)hy + (1.0f + M))), 0.0f) * grid.cy;
-        const float gz = fmaxf(fmaxf(((float)hz - M) - qz, qz - ((float)hz + (1.0f + M))), 0.0f) * grid.cz;
-        *near = !((gx * gx + gy * gy) + gz * gz > r_sq);
-        return h;
+        *lo = min(__ldg(&cs[h]), g.n_cap);
+        *hi = min(__ldg(&cs[h + 1]), g.n_cap);
     };
-    auto cell_photons = [&](u32 k, const u32 end) {
-        // PHX_GATHER_AHEAD records in flight per step; contributions still added in photon order
-#if PHX_GATHER_AHEAD == 4
-        for (; k + 3 < end; k += 4) {
-            const float4 p0 = __ldg(&g.s_posdir[k]);
-            const float4 p1 = __ldg(&g.s_posdir[k + 1]);
-            const float4 p2 = __ldg(&g.s_posdir[k + 2]);
-            const float4 p3 = __ldg(&g.s_posdir[k + 3]);
-            add(p0, k);
-            add(p1, k + 1);
-            add(p2, k + 2);
-            add(p3, k + 3);
+    u32 cnt = 0;
+    auto flush = [&]() {
+        for (u32 e = 0; __any_sync(FULL, e < cnt); e += GQ_BATCH) {
+            if (e >= cnt)
+                continue;
+            float4 pd[GQ_BATCH], pw[GQ_BATCH]; // decode_oct(p.w), decode_rgbe(s_power[k]), decoded once per round
+#pragma unroll
+            for (u32 u = 0; u < GQ_BATCH; u++) {
+                const u32 k = q_k[min(e + u, cnt - 1u)][tid];
+                pd[u] = __ldg(&g.s_dir[k]);
+                pw[u] = __ldg(&g.s_pow[k]);
+            }
+#pragma unroll
+            for (u32 u = 0; u < GQ_BATCH; u++) {
+                if (e + u < cnt && !((pd[u].x * nrm.x + pd[u].y * nrm.y) + pd[u].z * nrm.z > 0.0f)) { // both w are 0
+                    const float dsq = q_d[e + u][tid];
+                    const float x = (-GAUSS_BETA) * dsq;
+                    const float t = dsq >= dsq_min ? div_known(x, denom, rdenom) : x / denom;
+                    const float w = GAUSS_ALPHA * (1.0f - div_gauss(1.0f - exp_unit(t)));
+                    nf.x += w * pw[u].x;
+                    nf.y += w * pw[u].y;
+                    nf.z += w * pw[u].z;
+                    found += w;
+                }
+            }
         }
-#endif
-        for (; k + 1 < end; k += 2) {
-            const float4 p0 = __ldg(&g.s_posdir[k]);
-            const float4 p1 = __ldg(&g.s_posdir[k + 1]);
-            add(p0, k);
-            add(p1, k + 1);
-        }
-        if (k < end)
-            add(__ldg(&g.s_posdir[k]), k);
+        cnt = 0;
     };
-#if PHX_GATHER_NEXT_CELL
-    // Each cell's photon range is loaded while the previous cell's photons are summed: the scan for
-    // the next cell to search (each neighbour's hash computed once, as before) runs ahead by one.
-    auto next_cell = [&](u32 from, u32 *h) -> u32 {
-        for (u32 c = from; c < 27; c++) {
-            bool near;
-            *h = cell_of(c, &near);
-            if (near)
-                return c;
+    u32 k = 0, end = 0, n0 = 0, n1 = 0;
+    bool ahead = near != 0; // n0, n1: the range of the cell after the current one, loaded ahead
+    if (ahead)
+        next_cell(&n0, &n1);
+    for (;;) {
+        while (k >= end && ahead) { // the next cell with photons
+            k = n0;
+            end = n1;
+            ahead = near != 0;
+            if (ahead)
+                next_cell(&n0, &n1);
         }
-        return 27u;
-    };
-    u32 h = 0;
-    u32 i = next_cell(0, &h);
-    u32 k0 = 0, k1 = 0;
-    if (i < 27) {
-        k0 = __ldg(&cs[h]);
-        k1 = __ldg(&cs[h + 1]);
-    }
-    while (i < 27) {
-        u32 hn = 0, n0 = 0, n1 = 0;
-        const u32 j = next_cell(i + 1, &hn);
-        if (j < 27) {
-            n0 = __ldg(&cs[hn]);
-            n1 = __ldg(&cs[hn + 1]);
+        __syncwarp();
+        if (!__any_sync(FULL, k < end))
+            break;
+        if (k < end) {
+            float4 p[GQ_AHEAD];
+#pragma unroll
+            for (u32 u = 0; u < GQ_AHEAD; u++)
+                p[u] = __ldg(&g.s_posdir[min(k + u, end - 1u)]);
+#pragma unroll
+            for (u32 u = 0; u < GQ_AHEAD; u++) {
+                const float dx = pos.x - p[u].x, dy = pos.y - p[u].y, dz = pos.z - p[u].z;
+                const float dsq = ((dx * dx + dy * dy) + dz * dz) + dw * dw;
+                if (dsq < r_sq && k + u < end) {
+                    q_k[cnt][tid] = k + u;
+                    q_d[cnt][tid] = dsq;
+                    cnt++;
+                }
+            }
+            k += GQ_AHEAD;
         }
-        cell_photons(min(k0, g.n_cap), min(k1, g.n_cap));
-        i = j;
-        k0 = n0;
-        k1 = n1;
+        if (__any_sync(FULL, cnt > GQ_CAP - GQ_AHEAD))
+            flush();
     }
-#else
-    for (u32 i = 0; i < 27; i++) {
-        bool near;
-        const u32 h = cell_of(i, &near);
-        if (!near)
-            continue;
-        cell_photons(min(__ldg(&cs[h]), g.n_cap), min(__ldg(&cs[h + 1]), g.n_cap));
-    }
-#endif
+    flush();
+    if (!gathering)
+        return;
+    const float4 fso = g.flux[gpix];
+    const float wso = g.weight[gpix];
     if (g.rec_r2) {
         g.rec_r2[gpix] = r_sq;
         g.rec_ratio[gpix] = found > 0.0f ? (wso + sc.alpha * found) / (wso + found) : 1.0f;
@@ -192,22 +239,6 @@ PHX_DI void gather_pixel(const SceneDesc &sc, u32 gpix, const GatherBufs &g) {
     }
 }
 
-// 12 resident blocks per SM (42 registers, ~100 bytes of spills): the photon loop is latency-bound
-// and more warps hide it better (7.3 -> 6.4 ms; 16 blocks spill more and measured slower).
-#ifndef PHX_GATHER_MINB
-#define PHX_GATHER_MINB 12
-#endif
-__global__ void __launch_bounds__(128, PHX_GATHER_MINB) k_gather(LaunchCtx lc, GatherBufs g) {
-    u32 gid = blockIdx.x * blockDim.x + threadIdx.x;
-    if (gid >= lc.total_pixels)
-        return;
-    if (g.order)
-        gid = __ldg(&g.order[gid]);
-    u32 s = lc.n_scenes == 1 ? 0 : find_scene(lc.pix_bases, lc.n_scenes, gid);
-    if (lc.scenes[s].active)
-        gather_pixel(lc.scenes[s], gid, g);
-}
-
 // Cooperative form of the same gather.  The pixels arrive grouped by photon-grid cell (k_pixel_keys),
 // so the lanes of a warp mostly need the same cells.  For each of the 27 neighbour offsets the warp
 // forms groups of lanes that need the same (global) cell; for each group all 32 lanes load the
@@ -221,7 +252,7 @@ constexpr u32 COOP_WARPS = 4;
 #define PHX_GATHER_STAGE_ALL 1 // stage the decoded direction and power too (else load them per lane)
 #endif
 
-__global__ void __launch_bounds__(32 * COOP_WARPS, PHX_GATHER_MINB) k_gather_coop(LaunchCtx lc, GatherBufs g) {
+__global__ void __launch_bounds__(32 * COOP_WARPS, 12) k_gather_coop(LaunchCtx lc, GatherBufs g) {
     __shared__ float4 st_pd[COOP_WARPS][32];
 #if PHX_GATHER_STAGE_ALL
     __shared__ float4 st_dir[COOP_WARPS][32];

@@ -371,8 +371,9 @@ typedef struct phx_tuning {
     uint32_t emit_blocks_per_sm;
     uint32_t persistent;        /* 1 = persistent lane-refill kernels, 0 = one thread per item */
     uint32_t nee_wavefront;     /* 1 = diffuse-hit NEE shadow rays traced by a separate wavefront */
-    uint32_t concurrent_passes; /* 1 = in the captured graph the camera pass and the photon pass of a
-                                   round run on two branches (they only share the round seed) */
+    uint32_t concurrent_passes; /* 1 = a captured group of rounds (pipeline_rounds > 1) runs each round's
+                                   camera and photon passes on two branches (they only share the round
+                                   seed); rounds run one at a time always do */
     uint32_t gather_sorted;     /* 1 = the gather visits pixels grouped by photon-grid cell */
     uint32_t pipeline_rounds;   /* k > 1: graph replays capture k rounds at a time, each round's camera
                                    and photon passes on branches of their own (they depend only on

@@ -550,7 +550,6 @@ int Engine::create(const phx_scene *scenes, const phx_params *params, uint32_t n
         (r = radix_scr.alloc(radix_scratch_bytes(N, key_bits))))
         return r;
     perm = sv0.as<u32>();
-    rs0 = view_own_buffers();
     // gather order: sort the pixels by (cell, octant) key; needs the composite key to fit 32 bits
     pix_key_bits = key_bits + 3 <= 32 ? key_bits + 3 : 0;
     if (pix_key_bits) {
@@ -561,6 +560,7 @@ int Engine::create(const phx_scene *scenes, const phx_params *params, uint32_t n
             (r = upload(d_npix, &Pn, 4)))
             return r;
     }
+    rs0 = view_own_buffers();
     CK(cudaMallocHost((void **)&h_pinned, 4096));
     tune.trace_block = 128;
     tune.emit_block = 128;
@@ -653,6 +653,12 @@ RoundSet Engine::view_own_buffers() {
     R.s_pow = s_pow.as<float4>();
     R.scan_scr = scan_scr.p;
     R.radix_scr = radix_scr.p;
+    R.pk_keys = pk_keys.as<u32>();
+    R.pk_t0 = pk_t0.as<u32>();
+    R.pk_t1 = pk_t1.as<u32>();
+    R.pk_v0 = pk_v0.as<u32>();
+    R.pk_v1 = pk_v1.as<u32>();
+    R.pk_scr = pk_scr.p;
     R.perm = sv0.as<u32>();
     return R;
 }
@@ -723,7 +729,19 @@ void Engine::enq_trace_r(RoundSet &R, cudaStream_t s) {
     if (spec)
         launch_spec_resolve(l, o, s);
     ev(ST_SHADOW, true, s);
+    // the gather's pixel order needs the hit points alone, so it belongs to this branch of a round (timed
+    // stage by stage it is the gather's)
+    if (!profiling)
+        enq_order_r(R, s);
     stage_state |= 1;
+}
+
+void Engine::enq_order_r(RoundSet &R, cudaStream_t s) {
+    if (!tune.gather_sorted || !pix_key_bits)
+        return;
+    launch_pixel_keys(lc(R), R.hp[0], R.hp[5], pix_key_bits, R.pk_keys, s);
+    launch_radix_sort(R.pk_keys, R.pk_t0, R.pk_t1, R.pk_v0, R.pk_v1, &R.order, d_npix.as<u32>(), total_pixels,
+                      pix_key_bits, R.pk_scr, d_err.as<u32>(), s);
 }
 
 void Engine::enq_emit_r(RoundSet &R, cudaStream_t s) {
@@ -765,19 +783,31 @@ void Engine::enq_hash_sort_r(RoundSet &R, cudaStream_t s) {
 void Engine::enq_gather_r(RoundSet &R, cudaStream_t s) {
     adjoint_invalidate();
     ev(ST_GATHER, false, s);
-    const u32 *order = nullptr;
-    if (tune.gather_sorted && pix_key_bits) {
-        launch_pixel_keys(lc(R), R.hp[0], R.hp[5], pix_key_bits, pk_keys.as<u32>(), s);
-        launch_radix_sort(pk_keys.as<u32>(), pk_t0.as<u32>(), pk_t1.as<u32>(), pk_v0.as<u32>(), pk_v1.as<u32>(),
-                          &pix_order, d_npix.as<u32>(), total_pixels, pix_key_bits, pk_scr.p, d_err.as<u32>(), s);
-        order = pix_order;
-    }
+    if (profiling)
+        enq_order_r(R, s);
     GatherBufs g{R.hp[0], R.hp[1], R.hp[2], R.hp[3], R.hp[4], R.hp[5], R.s_posdir, R.s_power, R.s_dir, R.s_pow,
                  R.cell_start, (u32)max_photons, flux.as<float4>(), weight.as<float>(), radiance.as<float4>(), rec_r2,
-                 rec_ratio, order};
+                 rec_ratio, tune.gather_sorted ? R.order : nullptr};
     launch_gather(lc(R), g, (int)tune.gather_block, tune.gather_coop != 0, s);
     ev(ST_GATHER, true, s);
 }
+
+// The camera pass and the photon passes of a round share its seeds and nothing else, so in the forms that
+// run one round at a time the camera pass (with its shadow rays and the gather's pixel order) goes to a
+// stream of its own, from the seed step to the gather.  Not while stages are timed one by one.  Small rounds
+// are chains of short kernels, and the camera chain (with the pixel order, 135 of 365 us for a 64 x 64
+// view) then runs beside the photon one: 0.44 -> 0.31 ms a view, 2.41 -> 1.88 ms for two rounds of 333 x 251;
+// large ones overlap each other's tails (1920 x 1080 atrium round 5.9 -> 5.6 ms).
+bool Engine::fork_passes() const { return !profiling; }
+
+void Engine::enq_trace_side() {
+    cudaEventRecord(fork_ev, st);
+    cudaStreamWaitEvent(st_side, fork_ev, 0);
+    enq_trace_r(rs0, st_side);
+    cudaEventRecord(join_ev, st_side);
+}
+
+void Engine::join_side() { cudaStreamWaitEvent(st, join_ev, 0); }
 
 void Engine::enq_round() {
     enq_seeds();
@@ -928,22 +958,34 @@ int Engine::plain_round() {
     if (!any_active())
         return PHX_OK;
     enq_seeds();
-    enq_trace();
+    const bool fork = fork_passes();
+    if (fork)
+        enq_trace_side();
+    else
+        enq_trace();
     enq_emit();
     // renderer.cpp:113-118: blocking read of the stored-photon count
     uint32_t total = 0;
     int r = read_total(&total);
-    if (r)
+    if (r) {
+        if (fork)
+            join_side();
         return r;
+    }
     for (uint32_t s = 0; s < sc.size(); s++) {
         uint32_t off, n;
-        if ((r = scene_photon_range(s, &off, &n)))
+        r = scene_photon_range(s, &off, &n);
+        if (fork && (r || (n == 0 && sc[s].desc.active)))
+            join_side(); // whatever the stream does next waits for the camera pass
+        if (r)
             return r;
         if (n == 0 && sc[s].desc.active)
             return fail(PHX_E_NO_PHOTONS, "no photon hit (renderer.cpp:117-118)");
         sc[s].n_photons_last = n;
     }
     enq_hash_sort();
+    if (fork)
+        join_side();
     enq_gather();
     r = sync_and_check(); // renderer.cpp:160 queue.finish()
     if (r)
@@ -960,20 +1002,15 @@ int Engine::capture(bool with_seeds, cudaGraph_t *g, cudaGraphExec_t *ge) {
     capturing = true;
     if (with_seeds)
         enq_seeds();
-    if (tune.concurrent_passes) {
-        // the photon pass only shares the round seed with the camera pass: fork it onto a second
-        // branch of the graph and join before the hash stage
-        cudaEventRecord(fork_ev, st);
-        cudaStreamWaitEvent(st_side, fork_ev, 0);
-        enq_emit(st_side);
+    const bool fork = fork_passes();
+    if (fork)
+        enq_trace_side();
+    else
         enq_trace();
-        cudaEventRecord(join_ev, st_side);
-        cudaStreamWaitEvent(st, join_ev, 0);
-    } else {
-        enq_trace();
-        enq_emit();
-    }
+    enq_emit();
     enq_hash_sort();
+    if (fork)
+        join_side();
     enq_gather();
     capturing = false;
     cudaError_t e = cudaStreamEndCapture(st, g);
@@ -1009,7 +1046,7 @@ int Engine::alloc_round_sets(uint32_t sets) {
     const size_t P = total_pixels, E = total_emit, C = (size_t)total_cells + 1, N = max_photons,
                  NE = total_nee, n = sc.size();
     while (xsets.size() < sets) {
-        std::vector<DevBuf> b(44);
+        std::vector<DevBuf> b(50);
         RoundSet R;
         int k = 0, r = 0;
         auto get = [&](size_t bytes, bool zero) -> void * {
@@ -1056,6 +1093,14 @@ int Engine::alloc_round_sets(uint32_t sets) {
         R.s_pow = (float4 *)get(16 * N, true);
         R.scan_scr = get(std::max(scan_scratch_bytes(E + 1), scan_scratch_bytes(C)), false);
         R.radix_scr = get(radix_scratch_bytes(N, key_bits), false);
+        if (pix_key_bits) {
+            R.pk_keys = (u32 *)get(4 * P, false);
+            R.pk_t0 = (u32 *)get(4 * P, false);
+            R.pk_t1 = (u32 *)get(4 * P, false);
+            R.pk_v0 = (u32 *)get(4 * P, false);
+            R.pk_v1 = (u32 *)get(4 * P, false);
+            R.pk_scr = get(radix_scratch_bytes(P, pix_key_bits), false);
+        }
         R.perm = R.sv0;
         if (r) {
             for (auto &d : b)

@@ -93,6 +93,9 @@ struct RoundSet {
     float4 *s_dir = nullptr, *s_pow = nullptr;
     void *scan_scr = nullptr, *radix_scr = nullptr;
     u32 *perm = nullptr; // the photon sort's permutation (set by the hash stage)
+    u32 *pk_keys = nullptr, *pk_t0 = nullptr, *pk_t1 = nullptr, *pk_v0 = nullptr, *pk_v1 = nullptr;
+    void *pk_scr = nullptr;
+    u32 *order = nullptr; // the gather's pixel order (set by the camera pass)
 };
 
 float ray_reach(float geom, const phx_light *l, uint32_t n);
@@ -106,7 +109,10 @@ class Engine {
     // enqueue (no host sync) on the engine's buffers (set 0)
     void enq_seeds() { enq_seeds_r(rs0, st); }
     void enq_trace() { enq_trace_r(rs0, st); }
-    void enq_emit(cudaStream_t s = nullptr) { enq_emit_r(rs0, s ? s : st); } // nullptr: the engine's stream
+    void enq_emit() { enq_emit_r(rs0, st); }
+    bool fork_passes() const;
+    void enq_trace_side(); // the camera pass on the side stream, from what the engine's stream has done so far
+    void join_side();      // the engine's stream waits for it
     void enq_hash_sort() {
         enq_hash_sort_r(rs0, st);
         perm = rs0.perm;
@@ -180,6 +186,7 @@ class Engine {
     void enq_emit_r(RoundSet &R, cudaStream_t s);
     void enq_hash_sort_r(RoundSet &R, cudaStream_t s);
     void enq_gather_r(RoundSet &R, cudaStream_t s);
+    void enq_order_r(RoundSet &R, cudaStream_t s);
     RoundSet view_own_buffers();
     RoundSet rs0;
     // pipelined graph form: `pipe_k` rounds per captured graph, each round's passes on branches of
@@ -198,7 +205,7 @@ class Engine {
                      uint32_t *cell, uint64_t *slot);
     int scene_photon_range(uint32_t s, uint32_t *off, uint32_t *n);
     void ev(int stage, bool end, cudaStream_t s = nullptr);
-    cudaStream_t st_side = nullptr;          // second branch of a captured round (photon pass)
+    cudaStream_t st_side = nullptr;          // a round's camera pass, beside its photon passes
     cudaEvent_t fork_ev = nullptr, join_ev = nullptr;
     void accumulate_profile();
 
@@ -232,7 +239,6 @@ class Engine {
     // pixel order of the gather (pixels grouped by photon-grid cell)
     DevBuf pk_keys, pk_t0, pk_t1, pk_v0, pk_v1, pk_scr, d_npix;
     uint32_t pix_key_bits = 0; // 0: the gather runs in pixel order
-    u32 *pix_order = nullptr;
 
     u32 *perm = nullptr;
     u32 *h_pinned = nullptr;

@@ -210,7 +210,7 @@ int Engine::adjoint_backward(const float *dl_dimage, float *grad, uint32_t n_gra
                         hp[4].as<float4>(), hp[5].as<float4>(), s_posdir.as<float4>(), s_power.as<u32>(),
                         s_dir.as<float4>(), s_pow.as<float4>(), cell_start.as<u32>(), (u32)max_photons,
                         flux.as<float4>(), weight.as<float>(), radiance.as<float4>(), nullptr, nullptr,
-                        pix_order};
+                        rs0.order};
         launch_gather_adj(lc(), gbuf, ab, st);
         launch_trace_adj(lc(), ab, st);
         launch_emit_adj(lc(), ab, st);

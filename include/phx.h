@@ -375,10 +375,12 @@ typedef struct phx_tuning {
                                    camera and photon passes on two branches (they only share the round
                                    seed); rounds run one at a time always do */
     uint32_t gather_sorted;     /* 1 = the gather visits pixels grouped by photon-grid cell */
-    uint32_t pipeline_rounds;   /* k > 1: graph replays capture k rounds at a time, each round's camera
-                                   and photon passes on branches of their own (they depend only on
-                                   the round seed) and the gathers in round order, so rounds overlap;
-                                   k - 1 extra sets of per-round buffers (1..8, 1 = off) */
+    uint32_t pipeline_rounds;   /* k > 1: graph replays capture up to k rounds at a time, each round's
+                                   camera and photon passes on branches of their own (they depend only
+                                   on the round seed) and the gathers in round order, so rounds overlap;
+                                   up to k - 1 extra sets of per-round buffers (1..8, 1 = off; default 4
+                                   where three extra sets take at most 4 GB, else 2; fewer rounds are
+                                   captured where their sets do not fit) */
     uint32_t gather_coop;       /* 1 = a warp stages each cell's photon records in shared memory and its
                                    lanes that need the cell walk them; 0 = one thread per pixel */
     uint32_t reserved[1];

@@ -40,10 +40,11 @@ int DevBuf::alloc(size_t b) {
 }
 
 void DevBuf::release() {
-    if (p)
+    if (p && !view)
         cudaFree(p);
     p = nullptr;
     bytes = 0;
+    view = false;
 }
 
 Engine::~Engine() {
@@ -51,9 +52,8 @@ Engine::~Engine() {
         cudaStreamSynchronize(st);
     shard_release();
     invalidate_graph();
-    for (auto &v : xbufs)
-        for (auto &b : v)
-            b.release();
+    for (auto &b : xbufs)
+        b.release();
     for (auto s : pipe_st)
         if (s)
             cudaStreamDestroy(s);
@@ -71,7 +71,7 @@ Engine::~Engine() {
     for (auto &s : sc)
         for (auto &b : s.bufs)
             b.release();
-    DevBuf *all[] = {&d_desc, &d_pix_bases, &d_emit_bases, &d_nee_bases, &nee_ray, &nee_val, &stash_sn, &stash_rng,
+    DevBuf *all[] = {&own_arena, &d_desc, &d_pix_bases, &d_emit_bases, &d_nee_bases, &nee_ray, &nee_val, &stash_sn, &stash_rng,
                      &spec_ray, &spec_val,
                      &spec_org, &spec_pix, &spec_next, &def_cnt, &def_prefix, &def_val, &def_tag, &d_seeds, &d_rng,
                      &d_err, &d_ovf, &d_queue, &d_ntotal,
@@ -521,45 +521,67 @@ int Engine::create(const phx_scene *scenes, const phx_params *params, uint32_t n
     int r;
     if ((r = upload(d_desc, descs.data(), sizeof(SceneDesc) * n)) || (r = upload(d_pix_bases, pb.data(), 4 * pb.size())) ||
         (r = upload(d_emit_bases, eb.data(), 4 * eb.size())) || (r = upload(d_nee_bases, nb.data(), 4 * nb.size())) ||
-        (r = nee_ray.alloc(16 * (size_t)total_nee)) || (r = nee_val.alloc(16 * (size_t)total_nee)) ||
-        (r = stash_sn.alloc(16 * (size_t)total_pixels)) || (r = stash_rng.alloc(4 * (size_t)total_pixels)) ||
-        (r = spec_ray.alloc(16 * (size_t)total_nee)) || (r = spec_val.alloc(16 * (size_t)total_nee)) ||
-        (r = spec_org.alloc(16 * (size_t)total_nee)) || (r = spec_pix.alloc(4 * (size_t)total_nee)) ||
-        (r = upload(spec_next, nullptr, 16)) || (r = upload(def_cnt, nullptr, 4 * (size_t)total_pixels)) ||
-        (r = def_prefix.alloc(16 * (size_t)total_pixels)) ||
-        (r = def_val.alloc(16 * (size_t)DEF_MAX * total_pixels)) ||
-        (r = def_tag.alloc(4 * (size_t)DEF_MAX * total_pixels)) ||
         (r = upload(d_rng, rng.data(), 4 * n)) ||
         (r = upload(d_seeds, nullptr, 4 * n)) || (r = upload(d_err, nullptr, 16)) || (r = upload(d_ovf, nullptr, 16)) ||
-        (r = upload(d_queue, nullptr, 16)) || (r = upload(d_ntotal, nullptr, 16)))
+        (r = upload(d_queue, nullptr, 16)) || (r = upload(d_ntotal, nullptr, 16)) ||
+        (r = upload(spec_next, nullptr, 16)))
         return r;
-    const size_t P = total_pixels, E = total_emit, C = (size_t)total_cells + 1, N = max_photons;
-    for (auto &b : hp)
-        if ((r = upload(b, nullptr, 16 * P))) // ImageBuffers::alloc zero-fills (image.cpp:11-21)
-            return r;
-    if ((r = upload(flux, nullptr, 16 * P)) || (r = upload(weight, nullptr, 4 * P)) || (r = upload(radiance, nullptr, 16 * P)) ||
-        (r = slot_pos.alloc(16 * N)) || (r = slot_pd.alloc(8 * N)) || (r = upload(counts, nullptr, 4 * (E + 1))) ||
-        (r = upload(offsets, nullptr, 4 * (E + 1))) || (r = upload(ph_pos, nullptr, 16 * N)) ||
-        (r = upload(ph_pd, nullptr, 8 * N)) || (r = upload(keys, nullptr, 4 * N)) ||
-        (r = upload(cell_count, nullptr, 4 * C)) || (r = upload(cell_start, nullptr, 4 * C)) ||
-        (r = sk0.alloc(4 * N)) || (r = sk1.alloc(4 * N)) || (r = upload(sv0, nullptr, 4 * N)) ||
-        (r = upload(sv1, nullptr, 4 * N)) || (r = upload(s_posdir, nullptr, 16 * N)) ||
-        (r = upload(s_power, nullptr, 4 * N)) || (r = upload(s_dir, nullptr, 16 * N)) ||
-        (r = upload(s_pow, nullptr, 16 * N)) ||
-        (r = scan_scr.alloc(std::max(scan_scratch_bytes(E + 1), scan_scratch_bytes(C)))) ||
-        (r = radix_scr.alloc(radix_scratch_bytes(N, key_bits))))
-        return r;
-    perm = sv0.as<u32>();
     // gather order: sort the pixels by (cell, octant) key; needs the composite key to fit 32 bits
     pix_key_bits = key_bits + 3 <= 32 ? key_bits + 3 : 0;
+    const size_t P = total_pixels, E = total_emit, C = (size_t)total_cells + 1, N = max_photons, NE = total_nee;
+    // every per-pixel, per-path, per-photon and per-cell buffer in one allocation (zero: cleared, like
+    // ImageBuffers::alloc's, image.cpp:11-21)
+    struct Part {
+        DevBuf *b;
+        size_t bytes;
+        bool zero;
+    };
+    std::vector<Part> parts{
+        {&nee_ray, 16 * NE, false}, {&nee_val, 16 * NE, false}, {&stash_sn, 16 * P, false}, {&stash_rng, 4 * P, false},
+        {&spec_ray, 16 * NE, false}, {&spec_val, 16 * NE, false}, {&spec_org, 16 * NE, false},
+        {&spec_pix, 4 * NE, false}, {&def_prefix, 16 * P, false}, {&def_val, 16 * (size_t)DEF_MAX * P, false},
+        {&def_tag, 4 * (size_t)DEF_MAX * P, false}, {&slot_pos, 16 * N, false}, {&slot_pd, 8 * N, false},
+        {&sk0, 4 * N, false}, {&sk1, 4 * N, false},
+        {&scan_scr, std::max(scan_scratch_bytes(E + 1), scan_scratch_bytes(C)), false},
+        {&radix_scr, radix_scratch_bytes(N, key_bits), false}};
+    if (pix_key_bits) {
+        for (DevBuf *b : {&pk_keys, &pk_t0, &pk_t1, &pk_v0, &pk_v1})
+            parts.push_back({b, 4 * P, false});
+        parts.push_back({&pk_scr, radix_scratch_bytes(P, pix_key_bits), false});
+    }
+    const size_t first_zero = parts.size();
+    for (auto &b : hp)
+        parts.push_back({&b, 16 * P, true});
+    for (const Part &q : {Part{&flux, 16 * P, true}, Part{&weight, 4 * P, true}, Part{&radiance, 16 * P, true},
+                          Part{&def_cnt, 4 * P, true}, Part{&counts, 4 * (E + 1), true},
+                          Part{&offsets, 4 * (E + 1), true}, Part{&ph_pos, 16 * N, true}, Part{&ph_pd, 8 * N, true},
+                          Part{&keys, 4 * N, true}, Part{&cell_count, 4 * C, true}, Part{&cell_start, 4 * C, true},
+                          Part{&sv0, 4 * N, true}, Part{&sv1, 4 * N, true}, Part{&s_posdir, 16 * N, true},
+                          Part{&s_power, 4 * N, true}, Part{&s_dir, 16 * N, true}, Part{&s_pow, 16 * N, true}})
+        parts.push_back(q);
+    size_t total = 0, zero_from = 0;
+    for (size_t i = 0; i < parts.size(); i++) {
+        if (i == first_zero)
+            zero_from = total;
+        total += (parts[i].bytes + 255) & ~(size_t)255;
+    }
+    if ((r = own_arena.alloc(total)))
+        return r;
+    CK(cudaMemset(own_arena.as<char>() + zero_from, 0, total - zero_from));
+    size_t at = 0;
+    for (const Part &q : parts) {
+        q.b->release();
+        q.b->p = own_arena.as<char>() + at;
+        q.b->bytes = q.bytes;
+        q.b->view = true;
+        at += (q.bytes + 255) & ~(size_t)255;
+    }
     if (pix_key_bits) {
         const uint32_t Pn = total_pixels;
-        if ((r = pk_keys.alloc(4 * (size_t)Pn)) || (r = pk_t0.alloc(4 * (size_t)Pn)) ||
-            (r = pk_t1.alloc(4 * (size_t)Pn)) || (r = pk_v0.alloc(4 * (size_t)Pn)) ||
-            (r = pk_v1.alloc(4 * (size_t)Pn)) || (r = pk_scr.alloc(radix_scratch_bytes(Pn, pix_key_bits))) ||
-            (r = upload(d_npix, &Pn, 4)))
+        if ((r = upload(d_npix, &Pn, 4)))
             return r;
     }
+    perm = sv0.as<u32>();
     rs0 = view_own_buffers();
     CK(cudaMallocHost((void **)&h_pinned, 4096));
     tune.trace_block = 128;
@@ -572,7 +594,13 @@ int Engine::create(const phx_scene *scenes, const phx_params *params, uint32_t n
     tune.concurrent_passes = 0;
     tune.gather_sorted = 1;
     tune.gather_coop = 0; // the per-thread gather measured faster (caustic 2.28 vs 3.15 ms, atrium 3.52 vs 4.19)
-    tune.pipeline_rounds = 2; // two rounds in flight per graph replay (measured faster, bit-identical)
+    // Rounds in flight per graph replay: four where their three extra buffer sets take at most 4 GB, else
+    // two.  Smaller rounds leave more of the GPU idle: against two, 512 x 512 Cornell 0.84 -> 0.77 ms a
+    // round, 333 x 251 0.59 -> 0.50, sixteen small scenes 1.40 -> 1.26; the large workloads' sets take 3 to
+    // 10 GB each for 1 to 3 % (caustic 9.45 -> 9.2 ms, atrium 5.6 -> 5.4).
+    size_t set_bytes = 0;
+    alloc_round_sets(0, &set_bytes);
+    tune.pipeline_rounds = 3 * set_bytes <= (4ull << 30) ? 4 : 2;
     for (uint32_t i = 0; i < n; i++)
         if (params[i].flags & PHX_F_SIMPLE_TRAVERSAL)
             tune.persistent = 0;
@@ -844,17 +872,18 @@ void Engine::invalidate_graph() {
         cudaGraphExecDestroy(gexec_host);
     if (graph_host)
         cudaGraphDestroy(graph_host);
-    if (gexec_pipe)
-        cudaGraphExecDestroy(gexec_pipe);
-    if (graph_pipe)
-        cudaGraphDestroy(graph_pipe);
+    for (int k = 0; k <= MAX_PIPE; k++) {
+        if (gexec_pipe[k])
+            cudaGraphExecDestroy(gexec_pipe[k]);
+        if (graph_pipe[k])
+            cudaGraphDestroy(graph_pipe[k]);
+        gexec_pipe[k] = nullptr;
+        graph_pipe[k] = nullptr;
+    }
     gexec = nullptr;
     graph = nullptr;
     gexec_host = nullptr;
     graph_host = nullptr;
-    gexec_pipe = nullptr;
-    graph_pipe = nullptr;
-    pipe_k = 0;
 }
 
 void Engine::set_profiling(bool on) {
@@ -1037,25 +1066,29 @@ void Engine::count_round(uint32_t rounds) {
 uint32_t Engine::pipeline_rounds() const {
     if (tune.pipeline_rounds <= 1 || profiling || rec_r2 || shard.world > 1)
         return 1;
-    return std::min(tune.pipeline_rounds, 8u);
+    return std::min(std::min(tune.pipeline_rounds, (uint32_t)MAX_PIPE), pipe_fits);
 }
 
-// Allocates `sets` more sets of per-round buffers, sized like the engine's own (zero-filled where
-// those are).
-int Engine::alloc_round_sets(uint32_t sets) {
+// Allocates per-round buffers until there are `sets` sets besides the engine's own, sized like those
+// (zero-filled where those are).  A set is one allocation: forty separate ones took most of the first call's
+// time.  only_bytes: just the size of one set.
+int Engine::alloc_round_sets(uint32_t sets, size_t *only_bytes) {
     const size_t P = total_pixels, E = total_emit, C = (size_t)total_cells + 1, N = max_photons,
                  NE = total_nee, n = sc.size();
-    while (xsets.size() < sets) {
-        std::vector<DevBuf> b(50);
-        RoundSet R;
-        int k = 0, r = 0;
-        auto get = [&](size_t bytes, bool zero) -> void * {
-            DevBuf &d = b[k++];
-            if (r)
-                return nullptr;
-            r = zero ? upload(d, nullptr, bytes) : d.alloc(bytes);
-            return d.p;
-        };
+    RoundSet R;
+    DevBuf arena;
+    size_t off = 0;
+    bool zeroed = true;
+    // the buffers of R at their places in the arena (or, without one, only their total size)
+    auto get = [&](size_t bytes, bool zero) -> void * {
+        char *p = arena.p ? arena.as<char>() + off : nullptr;
+        off += (bytes + 255) & ~(size_t)255;
+        if (p && zero)
+            zeroed = cudaMemsetAsync(p, 0, bytes, st) == cudaSuccess && zeroed;
+        return p;
+    };
+    auto lay_out = [&]() {
+        off = 0;
         R.seeds = (u32 *)get(4 * n, true);
         R.queue = (u32 *)get(16, true);
         R.ntotal = (u32 *)get(16, true);
@@ -1102,13 +1135,26 @@ int Engine::alloc_round_sets(uint32_t sets) {
             R.pk_scr = get(radix_scratch_bytes(P, pix_key_bits), false);
         }
         R.perm = R.sv0;
-        if (r) {
-            for (auto &d : b)
-                d.release();
+        R.order = nullptr;
+    };
+    lay_out();
+    const size_t bytes = off;
+    if (only_bytes) {
+        *only_bytes = bytes;
+        return PHX_OK;
+    }
+    while (xsets.size() < sets) {
+        int r = arena.alloc(bytes);
+        if (r)
             return r;
+        lay_out();
+        if (!zeroed) {
+            arena.release();
+            return fail(PHX_E_CUDA, "clearing a round's buffers failed");
         }
-        xbufs.push_back(std::move(b));
+        xbufs.push_back(arena);
         xsets.push_back(R);
+        arena = DevBuf{};
     }
     return PHX_OK;
 }
@@ -1134,6 +1180,10 @@ int Engine::capture_pipelined(uint32_t k) {
         pipe_ev.push_back(e);
     }
     auto set = [&](uint32_t i) -> RoundSet & { return i == k - 1 ? rs0 : xsets[k - 2 - i]; };
+    // two rounds leave room for their camera and photon passes on branches of their own (1024 x 1024 caustic
+    // round 9.58 -> 9.45 ms, 1920 x 1080 atrium 5.88 -> 5.60, 333 x 251 0.69 -> 0.59); three and more fill the
+    // GPU without (640 x 361 textured atrium 0.93 ms against 1.07 with)
+    const bool branch = tune.concurrent_passes || k == 2;
     CK(cudaStreamSynchronize(st));
     CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
     capturing = true;
@@ -1143,7 +1193,7 @@ int Engine::capture_pipelined(uint32_t k) {
         cudaEventRecord(pipe_ev[3 * i], st); // round i's seeds
         cudaStream_t a = pipe_st[2 * i], b = pipe_st[2 * i + 1];
         cudaStreamWaitEvent(a, pipe_ev[3 * i], 0);
-        if (tune.concurrent_passes) {
+        if (branch) {
             cudaStreamWaitEvent(b, pipe_ev[3 * i], 0);
             enq_emit_r(R, b);
             enq_trace_r(R, a);
@@ -1162,13 +1212,12 @@ int Engine::capture_pipelined(uint32_t k) {
     }
     perm = rs0.perm;
     capturing = false;
-    cudaError_t e = cudaStreamEndCapture(st, &graph_pipe);
+    cudaError_t e = cudaStreamEndCapture(st, &graph_pipe[k]);
     if (e != cudaSuccess) {
-        graph_pipe = nullptr;
+        graph_pipe[k] = nullptr;
         return fail(PHX_E_CUDA, std::string("stream capture failed: ") + cudaGetErrorString(e));
     }
-    CK(cudaGraphInstantiate(&gexec_pipe, graph_pipe, 0));
-    pipe_k = k;
+    CK(cudaGraphInstantiate(&gexec_pipe[k], graph_pipe[k], 0));
     return PHX_OK;
 }
 
@@ -1179,32 +1228,28 @@ int Engine::graph_rounds(uint32_t rounds) {
     if (!any_active())
         return PHX_OK;
     int r;
-    const uint32_t k = pipeline_rounds();
-    uint32_t single = rounds;
-    if (k > 1 && rounds >= k) {
-        if (pipe_k != k) {
-            if (gexec_pipe)
-                cudaGraphExecDestroy(gexec_pipe);
-            if (graph_pipe)
-                cudaGraphDestroy(graph_pipe);
-            gexec_pipe = nullptr;
-            graph_pipe = nullptr;
-            pipe_k = 0;
-            if ((r = capture_pipelined(k)))
+    // whole groups of the tuning's size, then one group of what is left
+    for (uint32_t left = rounds; left > 0;) {
+        const uint32_t k = std::min(pipeline_rounds(), left);
+        if (k > 1) {
+            if (!gexec_pipe[k] && (r = capture_pipelined(k))) {
+                if (r != PHX_E_OOM)
+                    return r;
+                cudaGetLastError();
+                pipe_fits = k - 1; // the sets of this many rounds do not fit beside the rest
+                continue;
+            }
+            CK(cudaGraphLaunch(gexec_pipe[k], st));
+        } else {
+            if (!gexec && (r = capture(true, &graph, &gexec)))
                 return r;
+            CK(cudaGraphLaunch(gexec, st));
+            if (profiling) {
+                CK(cudaStreamSynchronize(st));
+                accumulate_profile();
+            }
         }
-        for (uint32_t i = 0; i < rounds / k; i++)
-            CK(cudaGraphLaunch(gexec_pipe, st));
-        single = rounds % k;
-    }
-    if (single && !gexec && (r = capture(true, &graph, &gexec)))
-        return r;
-    for (uint32_t i = 0; i < single; i++) {
-        CK(cudaGraphLaunch(gexec, st));
-        if (profiling) {
-            CK(cudaStreamSynchronize(st));
-            accumulate_profile();
-        }
+        left -= k;
     }
     r = sync_and_check();
     if (r)

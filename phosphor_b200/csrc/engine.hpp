@@ -23,6 +23,7 @@ namespace phx {
 struct DevBuf {
     void *p = nullptr;
     size_t bytes = 0;
+    bool view = false; // part of another allocation, not freed on its own
     int alloc(size_t b);
     void release();
     template <class T> T *as() const { return reinterpret_cast<T *>(p); }
@@ -189,18 +190,19 @@ class Engine {
     void enq_order_r(RoundSet &R, cudaStream_t s);
     RoundSet view_own_buffers();
     RoundSet rs0;
-    // pipelined graph form: `pipe_k` rounds per captured graph, each round's passes on branches of
+    // pipelined graph form: several rounds per captured graph, each round's passes on branches of
     // their own, the gathers in round order; extra buffer sets for all but the last round
     uint32_t pipeline_rounds() const;
-    int alloc_round_sets(uint32_t sets);
+    int alloc_round_sets(uint32_t sets, size_t *only_bytes = nullptr);
     int capture_pipelined(uint32_t k);
-    std::vector<std::vector<DevBuf>> xbufs;
+    std::vector<DevBuf> xbufs; // one per extra set
     std::vector<RoundSet> xsets;
     std::vector<cudaStream_t> pipe_st;
     std::vector<cudaEvent_t> pipe_ev;
-    cudaGraph_t graph_pipe = nullptr;
-    cudaGraphExec_t gexec_pipe = nullptr;
-    uint32_t pipe_k = 0;
+    static constexpr int MAX_PIPE = 8;
+    cudaGraph_t graph_pipe[MAX_PIPE + 1] = {}; // by group size
+    cudaGraphExec_t gexec_pipe[MAX_PIPE + 1] = {};
+    uint32_t pipe_fits = MAX_PIPE; // largest group whose buffer sets could be allocated
     int upload_scene(uint32_t i, const phx_scene &s, const phx_params &p, uint32_t *pix, uint32_t *emit,
                      uint32_t *cell, uint64_t *slot);
     int scene_photon_range(uint32_t s, uint32_t *off, uint32_t *n);
@@ -210,6 +212,7 @@ class Engine {
     void accumulate_profile();
 
     DevBuf d_desc, d_pix_bases, d_emit_bases, d_nee_bases, d_seeds, d_rng, d_err, d_ovf, d_queue, d_ntotal;
+    DevBuf own_arena; // most of the buffers below are parts of it
     DevBuf nee_ray, nee_val, stash_sn, stash_rng;
     // deferred specular NEE: sample slots (as many as the diffuse ones) and per-pixel term lists
     DevBuf spec_ray, spec_val, spec_org, spec_pix, spec_next, def_cnt, def_prefix, def_val, def_tag;

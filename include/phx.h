@@ -512,6 +512,11 @@ PHX_API int phx_median_filter(const int32_t *in, float *out, uint32_t width, uin
                               float *kernel_ms);
 PHX_API int phx_weighted_filter(const int32_t *in, float *out, const float *weights, uint32_t width, uint32_t height,
                                 uint32_t k, float *kernel_ms);
+/* The same filters (0 mean, 1 median, 2 weighted) with the result as doubles, which filters_gpu.py returns
+ * (its :128 widens the kernels' floats), and the image as int32 or (in_u8) as bytes: a caller with 8-bit
+ * pixels neither widens them first nor the result afterwards. */
+PHX_API int phx_filter_f64(int filter, const void *in, int in_u8, double *out, const float *weights, uint32_t width,
+                           uint32_t height, uint32_t k, float *kernel_ms);
 
 PHX_API const char *phx_last_error(void);
 PHX_API const char *phx_version(void);

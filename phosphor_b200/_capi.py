@@ -196,6 +196,7 @@ PROTOTYPES = [
     ("phx_mean_filter", C.c_int, [VP, VP, C.c_uint32, C.c_uint32, C.c_uint32, VP]),
     ("phx_median_filter", C.c_int, [VP, VP, C.c_uint32, C.c_uint32, C.c_uint32, VP]),
     ("phx_weighted_filter", C.c_int, [VP, VP, VP, C.c_uint32, C.c_uint32, C.c_uint32, VP]),
+    ("phx_filter_f64", C.c_int, [C.c_int, VP, C.c_int, VP, VP, C.c_uint32, C.c_uint32, C.c_uint32, VP]),
     ("phx_batch_set_active", C.c_int, [VP, C.c_uint32, C.c_int]),
     ("phx_shard", C.c_int, [VP, C.c_uint32, C.c_uint32]),
     ("phx_shard_begin", C.c_int, [VP, C.POINTER(C.c_uint32)]),

@@ -588,11 +588,11 @@ PHX_API int phx_scan_noalloc(const uint32_t *in, uint32_t *out, uint32_t n, uint
     });
 }
 
-static int filter_entry(int mode, const int32_t *in, float *out, const float *weights, uint32_t width,
-                        uint32_t height, uint32_t k, float *kernel_ms) {
+static int filter_entry(int mode, const void *in, bool in_u8, void *out, bool out_f64, const float *weights,
+                        uint32_t width, uint32_t height, uint32_t k, float *kernel_ms) {
     return guard([&]() -> int {
         std::string msg;
-        const int rc = denoise_filter(mode, in, out, weights, width, height, k, kernel_ms, msg);
+        const int rc = denoise_filter(mode, in, in_u8, out, out_f64, weights, width, height, k, kernel_ms, msg);
         if (rc == 1)
             return fail(PHX_E_INVALID, msg);
         if (rc == 3)
@@ -603,17 +603,24 @@ static int filter_entry(int mode, const int32_t *in, float *out, const float *we
 
 PHX_API int phx_mean_filter(const int32_t *in, float *out, uint32_t width, uint32_t height, uint32_t k,
                             float *kernel_ms) {
-    return filter_entry(0, in, out, nullptr, width, height, k, kernel_ms);
+    return filter_entry(0, in, false, out, false, nullptr, width, height, k, kernel_ms);
 }
 
 PHX_API int phx_median_filter(const int32_t *in, float *out, uint32_t width, uint32_t height, uint32_t k,
                               float *kernel_ms) {
-    return filter_entry(1, in, out, nullptr, width, height, k, kernel_ms);
+    return filter_entry(1, in, false, out, false, nullptr, width, height, k, kernel_ms);
 }
 
 PHX_API int phx_weighted_filter(const int32_t *in, float *out, const float *weights, uint32_t width, uint32_t height,
                                 uint32_t k, float *kernel_ms) {
-    return filter_entry(2, in, out, weights, width, height, k, kernel_ms);
+    return filter_entry(2, in, false, out, false, weights, width, height, k, kernel_ms);
+}
+
+PHX_API int phx_filter_f64(int filter, const void *in, int in_u8, double *out, const float *weights, uint32_t width,
+                           uint32_t height, uint32_t k, float *kernel_ms) {
+    if (filter < 0 || filter > 2)
+        return guard([&]() -> int { return fail(PHX_E_INVALID, "filter must be 0 (mean), 1 (median) or 2 (weighted)"); });
+    return filter_entry(filter, in, in_u8 != 0, out, true, weights, width, height, k, kernel_ms);
 }
 
 } // extern "C"

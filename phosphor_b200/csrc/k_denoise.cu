@@ -14,7 +14,11 @@
 // weights too.  Larger windows read the image through the read-only cache.
 #include "kernels.hpp"
 
+#include <algorithm>
+#include <system_error>
+#include <thread>
 #include <type_traits>
+#include <vector>
 
 namespace phx {
 
@@ -72,8 +76,10 @@ template <> struct Pow2<1> {
 // The image is staged as float for the sums (each value converted once: the same value the
 // kernels' per-use (float) conversion gives) and as int for the median.  The three channels are
 // summed together; each channel's additions keep the kernels' order.
-template <int MODE, bool TILED, int MK>
-__global__ void __launch_bounds__(BX *BY) k_filter(const int *__restrict__ in, float *__restrict__ out,
+// IN: int, or unsigned char (an 8-bit image: the same values in a quarter of the bytes).  OUT: float, or
+// double (the float result, widened where it is written).
+template <int MODE, bool TILED, int MK, class IN, class OUT>
+__global__ void __launch_bounds__(BX *BY) k_filter(const IN *__restrict__ in, OUT *__restrict__ out,
                                                    const float *__restrict__ weights, int width, int height, int k) {
     using T = typename std::conditional<MODE == F_MEDIAN, int, float>::type;
     __shared__ T tile[TILED ? TILE_H * TILE_W * 3 : 1];
@@ -87,7 +93,7 @@ __global__ void __launch_bounds__(BX *BY) k_filter(const int *__restrict__ in, f
             const int gy = y0 + ty;
             if (gy < 0 || gy >= height) // rows outside the image are never read
                 continue;
-            const int *src = in + ((size_t)gy * width + gxa) * 3;
+            const IN *src = in + ((size_t)gy * width + gxa) * 3;
             T *dst = tile + ty * TILE_W * 3 + skip;
             for (int i = threadIdx.x; i < rowlen; i += BX)
                 dst[i] = (T)__ldg(&src[i]);
@@ -163,14 +169,14 @@ __global__ void __launch_bounds__(BX *BY) k_filter(const int *__restrict__ in, f
         r[1] = s1;
         r[2] = s2;
     }
-    float *o = out + ((size_t)y * width + x) * 3;
+    OUT *o = out + ((size_t)y * width + x) * 3;
     o[0] = r[0];
     o[1] = r[1];
     o[2] = r[2];
 }
 
-template <int MODE, int MK> void launch_mode(const int *in, float *out, const float *w, int width, int height, int k,
-                                             cudaStream_t st) {
+template <int MODE, int MK, class IN, class OUT>
+void launch_mode(const IN *in, OUT *out, const float *w, int width, int height, int k, cudaStream_t st) {
     const dim3 block(BX, BY), grid((width + BX - 1) / BX, (height + BY - 1) / BY);
     if (k <= TILE_K)
         k_filter<MODE, true, MK><<<grid, block, 0, st>>>(in, out, w, width, height, k);
@@ -178,12 +184,50 @@ template <int MODE, int MK> void launch_mode(const int *in, float *out, const fl
         k_filter<MODE, false, MK><<<grid, block, 0, st>>>(in, out, w, width, height, k);
 }
 
+template <class IN, class OUT>
+void launch_filter(int mode, const IN *in, OUT *out, const float *w, int width, int height, int k, cudaStream_t st) {
+    if (mode == F_MEAN)
+        launch_mode<F_MEAN, 0>(in, out, nullptr, width, height, k, st);
+    else if (mode == F_WEIGHTED)
+        launch_mode<F_WEIGHTED, 0>(in, out, w, width, height, k, st);
+    else if (k == 0)
+        launch_mode<F_MEDIAN, 0>(in, out, nullptr, width, height, k, st);
+    else if (k == 1)
+        launch_mode<F_MEDIAN, 1>(in, out, nullptr, width, height, k, st);
+    else
+        launch_mode<F_MEDIAN, 2>(in, out, nullptr, width, height, k, st);
+}
+
 } // namespace
+
+// Touches every page of a result buffer of several megabytes from a few threads.  A caller's buffer is
+// usually fresh from the system, and the copy down then takes a page fault for each page on one thread:
+// 12 of 13 ms for the 50 MB of a 1920 x 1080 result.  Its contents are about to be overwritten.
+static void fault_in(void *p, size_t bytes) {
+    constexpr size_t PAGE = 4096, SHARE = (size_t)4 << 20;
+    const unsigned n = (unsigned)std::min<size_t>(std::min(8u, std::max(1u, std::thread::hardware_concurrency())),
+                                                  bytes / SHARE);
+    if (n < 2)
+        return;
+    std::vector<std::thread> threads;
+    const size_t share = (bytes / n + PAGE - 1) / PAGE * PAGE;
+    try {
+        for (unsigned t = 0; t < n; t++)
+            threads.emplace_back([=] {
+                volatile char *c = static_cast<char *>(p);
+                for (size_t i = t * share; i < std::min(bytes, (t + 1) * share); i += PAGE)
+                    c[i] = 0;
+            });
+    } catch (const std::system_error &) { // no more threads: the copy faults the rest in
+    }
+    for (auto &t : threads)
+        t.join();
+}
 
 // Runs one filter on host arrays: copies in, one kernel, copies out.  Returns 0, or 1 (invalid
 // argument) / 3 (CUDA error) with `msg` set; *kernel_ms (if given) is the kernel's CUDA-event time.
-int denoise_filter(int mode, const int32_t *in, float *out, const float *weights, uint32_t width, uint32_t height,
-                   uint32_t k, float *kernel_ms, std::string &msg) {
+int denoise_filter(int mode, const void *in, bool in_u8, void *out, bool out_f64, const float *weights,
+                   uint32_t width, uint32_t height, uint32_t k, float *kernel_ms, std::string &msg) {
     if (!in || !out || (mode == F_WEIGHTED && !weights)) {
         msg = "null buffer";
         return 1;
@@ -201,20 +245,21 @@ int denoise_filter(int mode, const int32_t *in, float *out, const float *weights
         return 1;
     }
     const size_t n = (size_t)width * height * 3, nw = (size_t)(2 * k + 1) * (2 * k + 1);
+    const size_t in_bytes = n * (in_u8 ? 1 : 4), out_bytes = n * (out_f64 ? 8 : 4);
     cudaStream_t st = nullptr;
-    int *d_in = nullptr;
-    float *d_out = nullptr, *d_w = nullptr;
+    void *d_in = nullptr, *d_out = nullptr;
+    float *d_w = nullptr;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     cudaError_t err = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
     auto ok = [&]() { return err == cudaSuccess; };
     if (ok())
-        err = cudaMallocAsync((void **)&d_in, n * sizeof(int), st);
+        err = cudaMallocAsync(&d_in, in_bytes, st);
     if (ok())
-        err = cudaMallocAsync((void **)&d_out, n * sizeof(float), st);
+        err = cudaMallocAsync(&d_out, out_bytes, st);
     if (ok() && mode == F_WEIGHTED)
         err = cudaMallocAsync((void **)&d_w, nw * sizeof(float), st);
     if (ok())
-        err = cudaMemcpyAsync(d_in, in, n * sizeof(int), cudaMemcpyHostToDevice, st);
+        err = cudaMemcpyAsync(d_in, in, in_bytes, cudaMemcpyHostToDevice, st);
     if (ok() && d_w)
         err = cudaMemcpyAsync(d_w, weights, nw * sizeof(float), cudaMemcpyHostToDevice, st);
     if (ok() && kernel_ms) {
@@ -226,22 +271,23 @@ int denoise_filter(int mode, const int32_t *in, float *out, const float *weights
     }
     if (ok()) {
         const int w = (int)width, h = (int)height, kk = (int)k;
-        if (mode == F_MEAN)
-            launch_mode<F_MEAN, 0>(d_in, d_out, nullptr, w, h, kk, st);
-        else if (mode == F_WEIGHTED)
-            launch_mode<F_WEIGHTED, 0>(d_in, d_out, d_w, w, h, kk, st);
-        else if (k == 0)
-            launch_mode<F_MEDIAN, 0>(d_in, d_out, nullptr, w, h, kk, st);
-        else if (k == 1)
-            launch_mode<F_MEDIAN, 1>(d_in, d_out, nullptr, w, h, kk, st);
+        auto go = [&](auto *i, auto *o) { launch_filter(mode, i, o, d_w, w, h, kk, st); };
+        if (in_u8 && out_f64)
+            go((const unsigned char *)d_in, (double *)d_out);
+        else if (in_u8)
+            go((const unsigned char *)d_in, (float *)d_out);
+        else if (out_f64)
+            go((const int *)d_in, (double *)d_out);
         else
-            launch_mode<F_MEDIAN, 2>(d_in, d_out, nullptr, w, h, kk, st);
+            go((const int *)d_in, (float *)d_out);
         err = cudaGetLastError();
     }
     if (ok() && kernel_ms)
         err = cudaEventRecord(e1, st);
-    if (ok())
-        err = cudaMemcpyAsync(out, d_out, n * sizeof(float), cudaMemcpyDeviceToHost, st);
+    if (ok()) {
+        fault_in(out, out_bytes); // while the image goes up and the kernel runs
+        err = cudaMemcpyAsync(out, d_out, out_bytes, cudaMemcpyDeviceToHost, st);
+    }
     if (ok())
         err = cudaStreamSynchronize(st);
     if (ok() && kernel_ms)

@@ -112,8 +112,8 @@ int selftest_lookback_timeout(int device, u32 n, u32 *err_out);
 // returns 0 ok, 1 too large, 3 CUDA error, 4 look-back timeout (message in err)
 int scan_noalloc(const u32 *in, u32 *out, u32 n, u32 *total, cudaStream_t st, std::string &err);
 // k_denoise.cu: mode 0 mean, 1 median, 2 weighted; 0 = ok, 1 = invalid argument, 3 = CUDA error
-int denoise_filter(int mode, const int32_t *in, float *out, const float *weights, uint32_t width, uint32_t height,
-                   uint32_t k, float *kernel_ms, std::string &msg);
+int denoise_filter(int mode, const void *in, bool in_u8, void *out, bool out_f64, const float *weights,
+                   uint32_t width, uint32_t height, uint32_t k, float *kernel_ms, std::string &msg);
 
 // k_bvh.cu: the binned-SAH traversal tree built on the device, identical to the host builder's
 // (bvh_build_sah, then bvh_widen when `widen`).  Topology first; bvh_device_finish then orders each

@@ -4,7 +4,7 @@ Same names, arguments, results and errors as filters_gpu.py, so denoise.py's men
 (Mean3/5, Median3/5, Gaussian3_1 ... 5_2) run unchanged against this module:
 
 * mean_filter_gpu(arr, k=1), median_filter_gpu(arr, k=1), gaussian_filter_gpu(arr, k=1, sd=1):
-  arr is an (H, W, 3) array, taken as int32 like filters_gpu.py:_run_kernel; the result is an
+  arr is an (H, W, 3) array, taken as int32 like filters_gpu.py:_run_kernel (8-bit images as they are); the result is an
   (H, W, 3) float64 array of the kernel's float32 values (filters_gpu.py:128);
 * ValueError for an array that is not (H, W, 3) and for a median with k > 2 (filters_gpu.py:116-117,
   138-139); other failures raise phosphor_b200's PhxError.
@@ -28,37 +28,39 @@ def last_kernel_ms() -> float:
     return _last_ms[0]
 
 
-def _run(fn: str, arr, k: int, weights: np.ndarray | None = None) -> np.ndarray:
+_MEAN, _MEDIAN, _WEIGHTED = 0, 1, 2
+
+
+def _run(filter_: int, arr, k: int, weights: np.ndarray | None = None) -> np.ndarray:
+    """One filter through phx_filter_f64.  8-bit images go up as they are and the float64 result comes
+    straight down: widening on the host both ways touched 100 MB of fresh memory for a 1920x1080 image,
+    most of the call's time (15-25 ms)."""
     a = np.asarray(arr)
     if a.ndim != 3 or a.shape[2] != 3:
         raise ValueError("expected an (H, W, 3) array")
     h, w, _ = a.shape
-    src = np.ascontiguousarray(a.astype(np.int32))
-    out = np.empty((h, w, 3), dtype=np.float32)
+    u8 = a.dtype == np.uint8
+    src = np.ascontiguousarray(a if u8 else a.astype(np.int32))
+    out = np.empty((h, w, 3), dtype=np.float64)
     ms = C.c_float(0.0)
-    lib = A.load()
-    if weights is None:
-        rc = getattr(lib, fn)(src.ctypes.data_as(C.c_void_p), out.ctypes.data_as(C.c_void_p), w, h, int(k),
-                              C.byref(ms))
-    else:
-        wt = np.ascontiguousarray(weights, np.float32)
-        rc = getattr(lib, fn)(src.ctypes.data_as(C.c_void_p), out.ctypes.data_as(C.c_void_p),
-                              wt.ctypes.data_as(C.c_void_p), w, h, int(k), C.byref(ms))
-    A.check(rc)
+    wt = None if weights is None else np.ascontiguousarray(weights, np.float32)
+    A.check(A.load().phx_filter_f64(filter_, src.ctypes.data_as(C.c_void_p), int(u8), out.ctypes.data_as(C.c_void_p),
+                                    None if wt is None else wt.ctypes.data_as(C.c_void_p), w, h, int(k),
+                                    C.byref(ms)))
     _last_ms[0] = ms.value
-    return out.astype(np.float64)
+    return out
 
 
 def mean_filter_gpu(arr, k=1):
     """filters_gpu.py:131-133 (kernel :9-27): the mean of each pixel's clamped window."""
-    return _run("phx_mean_filter", arr, k)
+    return _run(_MEAN, arr, k)
 
 
 def median_filter_gpu(arr, k=1):
     """filters_gpu.py:136-141 (kernel :29-67): the median of each pixel's clamped window, k <= 2."""
     if k > 2:
         raise ValueError("median filter k is > 3")
-    return _run("phx_median_filter", arr, k)
+    return _run(_MEDIAN, arr, k)
 
 
 def gaussian(x, y, sd):
@@ -81,7 +83,7 @@ def gaussian_weights(k: int = 1, sd: float = 1) -> np.ndarray:
 def gaussian_filter_gpu(arr, k=1, sd=1):
     """filters_gpu.py:146-161 (kernel :69-86): the Gaussian-weighted sum of each clamped window
     (the weights are not renormalised where a border window shrinks, as in the reference)."""
-    return _run("phx_weighted_filter", arr, k, gaussian_weights(k, sd))
+    return _run(_WEIGHTED, arr, k, gaussian_weights(k, sd))
 
 
 def bench(width: int = 1920, height: int = 1080, reps: int = 5) -> list[dict]:

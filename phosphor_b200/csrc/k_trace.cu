@@ -494,6 +494,7 @@ PHX_DI bool cp_advance(CameraPath &p, bool hit, const Hit &h, const TraceOut &ou
         cp_finish(p, out, false);
         return false;
     }
+    const u32 lanes = __activemask();
     phx_material mat = sc.materials[tri_mat(sc, h.tri)];
     if constexpr (NOTEX)
         mat.diff_index = mat.emis_index = mat.norm_index = mat.occlusion_index = mat.metal_rough_index =
@@ -519,13 +520,11 @@ PHX_DI bool cp_advance(CameraPath &p, bool hit, const Hit &h, const TraceOut &ou
     p.bs_thr = bs.throughput;
     p.nee_sum = zero4();
     p.nee_i = 0;
+    const bool stashed = bs.event == BSDF_DIFFUSE && defer;
     if (bs.event == BSDF_DIFFUSE) {
         p.nee_kind = NEE_DIFFUSE;
-        if (defer) {
+        if (stashed)
             stash_nee(out, p.gpix, p.rng, p.sn);
-            cp_finish(p, out, true, true);
-            return false;
-        }
     } else if (bs.event == BSDF_METALLIC) {
         p.nee_kind = NEE_SPECULAR;
         p.f0 = ctx.base_color;
@@ -536,13 +535,18 @@ PHX_DI bool cp_advance(CameraPath &p, bool hit, const Hit &h, const TraceOut &ou
         p.f0 = f4(r0, r0, r0, 0.0f);
     } else {
         p.nee_kind = NEE_NONE;
-        return cp_continue(p, out);
     }
-    if (defer && out.spec_ray && cp_defer_specular(p, out))
-        return cp_continue(p, out);
-    if (cp_next_shadow(p))
+    bool listed = p.nee_kind == NEE_NONE; // nothing to trace here: the path goes on
+    if (p.nee_kind == NEE_SPECULAR && defer && out.spec_ray)
+        listed = cp_defer_specular(p, out);
+    __syncwarp(lanes);
+    if (stashed) {
+        cp_finish(p, out, true, true);
+        return false;
+    }
+    if (!listed && cp_next_shadow(p))
         return true;
-    return cp_after_nee(p, out);
+    return listed ? cp_continue(p, out) : cp_after_nee(p, out);
 }
 
 template <bool NOTEX>

@@ -195,6 +195,8 @@ class Engine {
     uint32_t pipeline_rounds() const;
     int alloc_round_sets(uint32_t sets, size_t *only_bytes = nullptr);
     int capture_pipelined(uint32_t k);
+    bool halved_grids = false; // while capturing a group of three or more rounds
+    uint32_t shared_blocks(uint32_t per_sm) const { return halved_grids ? (per_sm + 1) / 2 : per_sm; }
     std::vector<DevBuf> xbufs; // one per extra set
     std::vector<RoundSet> xsets;
     std::vector<cudaStream_t> pipe_st;

@@ -270,7 +270,7 @@ void launch_emit(const LaunchCtx &lc, const EmitOut &out, int block, int persist
         cudaMemsetAsync(queue, 0, sizeof(u32), st);
         if (prestart)
             k_emit_start<<<(lc.emit_hi - lc.emit_lo + 127) / 128, 128, 0, st>>>(lc, out);
-        int grid = g_sm_count * (blocks_per_sm > 0 ? blocks_per_sm : 8);
+        const int grid = refill_grid(lc.emit_hi - lc.emit_lo, blocks_per_sm);
         if (out.slot_pow) { // the adjoint's rounds
             if (untextured && prestart)
                 k_emit_persistent<true, true, true><<<grid, 128, 0, st>>>(lc, out, queue);

@@ -857,7 +857,7 @@ void launch_trace(const LaunchCtx &lc, const TraceOut &out, int block, int persi
         return;
     if (persistent && queue) {
         cudaMemsetAsync(queue, 0, sizeof(u32), st);
-        int grid = g_sm_count * (blocks_per_sm > 0 ? blocks_per_sm : 8);
+        const int grid = refill_grid(lc.pix_hi - lc.pix_lo, blocks_per_sm);
         if (untextured) // camera kernel 2.77 -> 2.44 ms (atrium), 1.04 -> 0.90 ms (caustic)
             k_trace_persistent<true><<<grid, 128, 0, st>>>(lc, out, queue);
         else

@@ -78,7 +78,7 @@ Engine::~Engine() {
                      &flux, &weight, &radiance, &slot_pos, &slot_pd, &counts, &offsets, &ph_pos, &ph_pd, &keys,
                      &cell_count, &cell_start, &sk0, &sk1, &sv0, &sv1, &s_posdir, &s_power, &s_dir, &s_pow, &scan_scr, &radix_scr,
                      &img_rgb, &img_ldr, &pk_keys, &pk_t0, &pk_t1, &pk_v0, &pk_v1, &pk_scr, &d_npix, &adj_seeds, &adj_r2, &adj_ratio, &adj_k, &adj_img, &adj_g, &adj_gT,
-                     &adj_gA, &adj_gphi, &adj_slot_pow, &adj_ph_pow, &adj_grad};
+                     &adj_gA, &adj_gphi, &adj_slot_pow, &adj_ph_pow, &adj_grad, &adj_paths};
     for (auto *b : all)
         b->release();
     for (auto &b : hp)

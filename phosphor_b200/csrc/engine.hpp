@@ -234,7 +234,7 @@ class Engine {
     int shard_phase = 0;
     // adjoint state: per round seeds, search radii² and SPPM ratios of the forward pass
     DevBuf adj_seeds, adj_r2, adj_ratio, adj_k, adj_img, adj_g, adj_gT, adj_gA, adj_gphi, adj_slot_pow, adj_ph_pow,
-        adj_grad;
+        adj_grad, adj_paths;
     uint32_t adj_rounds = 0;
     bool adj_ready = false, adj_k_ready = false, in_adjoint = false;
     static constexpr uint32_t ADJ_NO_ROUND = 0xffffffffu;

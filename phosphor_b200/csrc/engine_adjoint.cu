@@ -156,7 +156,7 @@ int Engine::adjoint_backward(const float *dl_dimage, float *grad, uint32_t n_gra
     if ((r = ensure(adj_g, 16 * (size_t)P)) || (r = ensure(adj_gT, 16 * (size_t)P)) ||
         (r = ensure(adj_gA, 16 * (size_t)P)) || (r = ensure(adj_gphi, 16 * max_photons)) ||
         (r = ensure(adj_slot_pow, 16 * total_slots)) || (r = ensure(adj_ph_pow, 16 * max_photons)) ||
-        (r = ensure(adj_grad, 8 * (size_t)std::max(np, 1u))))
+        (r = ensure(adj_grad, 8 * (size_t)std::max(np, 1u))) || (r = ensure(adj_paths, 4 * ((size_t)total_emit + 1))))
         return r;
     CK(cudaStreamSynchronize(st));
     // the image buffer is free after the forward pass
@@ -176,6 +176,8 @@ int Engine::adjoint_backward(const float *dl_dimage, float *grad, uint32_t n_gra
     ab.ph_pow = adj_ph_pow.as<float4>();
     ab.offsets = offsets.as<u32>();
     ab.grad = adj_grad.as<double>();
+    ab.paths = adj_paths.as<u32>();
+    ab.n_paths = adj_paths.as<u32>() + total_emit;
     ab.n_params = np;
     ab.n_mat = (u32)S.mats.size();
     ab.inv_rounds = 1.0f / (float)R;
@@ -194,9 +196,10 @@ int Engine::adjoint_backward(const float *dl_dimage, float *grad, uint32_t n_gra
             break;
         }
         if (n != live) {
-            enq_trace();
+            enq_trace_side();
             enq_emit();
             enq_hash_sort();
+            join_side();
         }
         adj_live = n;
         // the photons' unquantised power, in canonical order like the photons
@@ -212,8 +215,13 @@ int Engine::adjoint_backward(const float *dl_dimage, float *grad, uint32_t n_gra
                         flux.as<float4>(), weight.as<float>(), radiance.as<float4>(), nullptr, nullptr,
                         rs0.order};
         launch_gather_adj(lc(), gbuf, ab, st);
+        // the two replays share nothing but the gradient they add to
+        cudaEventRecord(fork_ev, st);
+        cudaStreamWaitEvent(st_side, fork_ev, 0);
+        launch_emit_adj(lc(), ab, st_side);
+        cudaEventRecord(join_ev, st_side);
         launch_trace_adj(lc(), ab, st);
-        launch_emit_adj(lc(), ab, st);
+        join_side();
         if (cudaGetLastError() != cudaSuccess)
             r = fail(PHX_E_CUDA, "adjoint kernel launch failed");
     }

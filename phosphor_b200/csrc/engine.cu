@@ -778,7 +778,7 @@ void Engine::enq_emit_r(RoundSet &R, cudaStream_t s) {
         adj_live = ADJ_NO_ROUND;
     EmitOut o{R.slot_pos, R.slot_pd, R.counts, in_adjoint ? adj_slot_pow.as<float4>() : nullptr};
     launch_emit(lc(R), o, (int)tune.emit_block, (int)tune.persistent, (int)shared_blocks(tune.emit_blocks_per_sm), R.queue + 1,
-                untextured(), photon_prestart(), s);
+                untextured(), photon_prestart(), rough(), s);
     ev(ST_EMIT, true, s);
     ev(ST_EMIT_SCAN, false, s);
     launch_scan(R.counts, R.offsets, (u64)total_emit + 1, R.scan_scr, R.ntotal, d_err.as<u32>(), s);
@@ -954,6 +954,20 @@ bool Engine::untextured() const {
                 m.transmission_index != PHX_NO_TEXTURE)
                 return false;
     return true;
+}
+
+// Whether the mean over the scenes of their materials' mean roughness is 0.6 or more: between the
+// workloads that gain from searching the microfacet attempts (boxes with walls of roughness 1, with and
+// without glass: 0.71 and up; mixed batches: 0.7) and those that lose (atriums: 0.47).
+bool Engine::rough() const {
+    double sum = 0.0;
+    for (const auto &s : sc) {
+        double m = 0.0;
+        for (const auto &mat : s.mats)
+            m += mat.roughness;
+        sum += m / (double)s.mats.size();
+    }
+    return sum >= 0.6 * (double)sc.size();
 }
 
 bool Engine::photon_prestart() const {

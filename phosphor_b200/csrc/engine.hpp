@@ -154,6 +154,7 @@ class Engine {
     bool any_active() const;
     bool untextured() const; // no material of any scene has a texture (indices are fixed at set-up)
     bool one_sample() const; // a hit point's NEE samples are all the same ray
+    bool rough() const;      // its surfaces are mostly rough (the photon kernel's microfacet sampler)
     bool photon_prestart() const; // every scene keeps >= 3 photon slots per path (k_emit_start)
 
     // differentiation (single-scene engines; engine_adjoint.cu)

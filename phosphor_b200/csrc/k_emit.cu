@@ -160,7 +160,7 @@ __global__ void __launch_bounds__(128) k_emit_start(LaunchCtx lc, EmitOut out) {
 // Consumes the pending query; returns true while the path continues.  NOTEX: no material of the
 // context has a texture (texture indices never change after set-up), so every texture branch is
 // compiled out of this instance.  POW: the stored photons' unquantised power is kept too (out.slot_pow).
-template <bool NOTEX, bool POW>
+template <bool NOTEX, bool POW, bool ROUGH>
 PHX_DI bool pp_advance(PhotonPath &p, bool hit, const Hit &h, const EmitOut &out) {
     const SceneDesc &sc = *p.sc;
     if (!hit)
@@ -198,7 +198,8 @@ PHX_DI bool pp_advance(PhotonPath &p, bool hit, const Hit &h, const EmitOut &out
     if (ended)
         return false;
     float4 view = -p.dir;
-    BsdfSample bs = sample_bsdf(&p.rng, ctx, ctx.shading_normal, sh.normal, view, &p.ior, sh.front_face);
+    float4 half;
+    BsdfSample bs = sample_bsdf_h<ROUGH>(&p.rng, ctx, ctx.shading_normal, sh.normal, view, &p.ior, sh.front_face, &half);
     if (bs.event == BSDF_DIFFUSE && dot(p.dir, sh.normal) < 0.0f) {
         out.slot_pos[p.slot] = sh.position;
         out.slot_pd[p.slot] = make_uint2(encode_rgbe(p.power), encode_oct(p.dir));
@@ -216,7 +217,7 @@ PHX_DI bool pp_advance(PhotonPath &p, bool hit, const Hit &h, const EmitOut &out
     return p.depth < sc.max_bounces;
 }
 
-template <bool NOTEX, bool PRE, bool POW = false>
+template <bool NOTEX, bool PRE, bool POW = false, bool ROUGH = false>
 __global__ void __launch_bounds__(128, PHX_EMIT_MINB) k_emit_persistent(LaunchCtx lc, EmitOut out, u32 *queue) {
     const u32 lane = threadIdx.x & 31u;
     const u32 lt_mask = (1u << lane) - 1u;
@@ -252,7 +253,7 @@ __global__ void __launch_bounds__(128, PHX_EMIT_MINB) k_emit_persistent(LaunchCt
         if (active) {
             Hit h;
             const bool hit = intersect(*p.sc, p.origin, p.dir, EPS, INF, &h, &ovf);
-            if (!pp_advance<NOTEX, POW>(p, hit, h, out)) {
+            if (!pp_advance<NOTEX, POW, ROUGH>(p, hit, h, out)) {
                 out.counts[p.gid] = p.n_out;
                 active = false;
             }
@@ -263,7 +264,7 @@ __global__ void __launch_bounds__(128, PHX_EMIT_MINB) k_emit_persistent(LaunchCt
 }
 
 void launch_emit(const LaunchCtx &lc, const EmitOut &out, int block, int persistent, int blocks_per_sm, u32 *queue,
-                 bool untextured, bool prestart, cudaStream_t st) {
+                 bool untextured, bool prestart, bool rough, cudaStream_t st) {
     if (lc.emit_hi <= lc.emit_lo)
         return;
     if (persistent && queue) {
@@ -272,7 +273,9 @@ void launch_emit(const LaunchCtx &lc, const EmitOut &out, int block, int persist
             k_emit_start<<<(lc.emit_hi - lc.emit_lo + 127) / 128, 128, 0, st>>>(lc, out);
         const int grid = refill_grid(lc.emit_hi - lc.emit_lo, blocks_per_sm);
         if (out.slot_pow) { // the adjoint's rounds
-            if (untextured && prestart)
+            if (untextured && prestart && rough)
+                k_emit_persistent<true, true, true, true><<<grid, 128, 0, st>>>(lc, out, queue);
+            else if (untextured && prestart)
                 k_emit_persistent<true, true, true><<<grid, 128, 0, st>>>(lc, out, queue);
             else if (prestart)
                 k_emit_persistent<false, true, true><<<grid, 128, 0, st>>>(lc, out, queue);
@@ -281,7 +284,9 @@ void launch_emit(const LaunchCtx &lc, const EmitOut &out, int block, int persist
             return;
         }
         // untextured: emit 4.52 -> 4.44 ms (caustic), 2.82 -> 2.73 ms (atrium)
-        if (untextured && prestart)
+        if (untextured && prestart && rough)
+            k_emit_persistent<true, true, false, true><<<grid, 128, 0, st>>>(lc, out, queue);
+        else if (untextured && prestart)
             k_emit_persistent<true, true><<<grid, 128, 0, st>>>(lc, out, queue);
         else if (untextured)
             k_emit_persistent<true, false><<<grid, 128, 0, st>>>(lc, out, queue);

@@ -82,9 +82,10 @@ struct EmitOut {
 };
 // untextured: no material of the context has a texture.  prestart: every scene has at least three
 // photon slots per path (max_bounces >= 3), so the lane-refill form can draw the paths' light
-// samples in a pre-pass (k_emit_start) and keep them in those slots.
+// samples in a pre-pass (k_emit_start) and keep them in those slots.  rough: the scenes' surfaces are mostly
+// rough, where microfacet attempts are worth searching (ggx_sample_vndf_tbn).
 void launch_emit(const LaunchCtx &lc, const EmitOut &out, int block, int persistent, int blocks_per_sm, u32 *queue,
-                 bool untextured, bool prestart, cudaStream_t st);
+                 bool untextured, bool prestart, bool rough, cudaStream_t st);
 
 // grid build
 struct GridBufs {

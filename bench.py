@@ -52,13 +52,13 @@ METRIC = "Mphotons/s"
 # ncu capture of one whole round of the caustic workload at 1/2 resolution and 1/4 photons (512x512
 # pixels, 2^18 photon paths, ~425k stored photons), scaled by 4 to the full workload (pixels for
 # trace_rays, photon paths or stored photons for the others; the 125,001-cell scan does not scale).
-# trace_rays = k_trace_persistent 220.3 MB + k_shadow 105.9 + k_nee_resolve 76.3 + k_spec_resolve
-# 13.3; emit_photons = k_emit_persistent 103.5 + k_emit_start 0.05 + k_scan 1.1 + k_compact 29.4;
-# scatter_photons = the two radix passes 9.5 + k_sorted_records 11.9; gather_flux = k_pixel_keys 8.3
-# + the pixel radix sort 6.4 + k_gather 58.7.  The integer stages' arrays stay in the 126 MB L2
+# trace_rays = k_trace_persistent 137.2 MB + k_shadow 91.2 + k_nee_resolve 76.1 + k_spec_resolve
+# 13.4; emit_photons = k_emit_persistent 108.5 + k_emit_start 0.04 + k_scan 1.1 + k_compact 28.7;
+# scatter_photons = the two radix passes 9.5 + k_sorted_records 12.0; gather_flux = k_pixel_keys 8.3
+# + the pixel radix sort 6.4 + k_gather 56.5.  The integer stages' arrays stay in the 126 MB L2
 # between kernels, so their DRAM bytes fall below the compulsory bytes.
-NCU_TRAFFIC: dict = {"caustic": {"trace_rays": 1663.3e6, "emit_photons": 536.2e6, "hash_photons": 28.2e6,
-                                 "scan": 0.51e6, "scatter_photons": 85.6e6, "gather_flux": 293.8e6}}
+NCU_TRAFFIC: dict = {"caustic": {"trace_rays": 1271.5e6, "emit_photons": 553.1e6, "hash_photons": 28.4e6,
+                                 "scan": 0.51e6, "scatter_photons": 85.9e6, "gather_flux": 284.8e6}}
 
 
 def load_peaks() -> tuple[float, str]:

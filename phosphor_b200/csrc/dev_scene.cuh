@@ -12,8 +12,9 @@
 // the current closest hit.  The reference's depth-first left-first order (hit.h:135-172) keeps
 // the LAST tested triangle among hits at exactly equal t (`t > t_max` rejects, equality passes,
 // hit.h:68); with left-first pre-order that is the equal-t hit with the largest leaf rank, so an
-// equal-t candidate replaces the current hit only when its rank is larger.  Boxes are expanded by
-// 1e-3 (bounding_box.h:30-37), so no box that holds the closest hit is ever culled by either
+// equal-t candidate replaces the current hit only when its rank is larger.  Boxes are expanded past
+// the triangle test's and the slab test's rounding (bvh_margin.hpp; at most the reference's 1e-3,
+// bounding_box.h:30-37), so no box that holds the closest hit is ever culled by either
 // order, and the result is the reference's hit for every ray.  The reference drops children when
 // its 24-entry stack is full (hit.h:163-164), which only happens for trees deeper than 22 levels;
 // the host reports the depth and this traversal counts (instead of silently dropping) overflows
@@ -161,7 +162,7 @@ PHX_DI void hit_uv(const SceneDesc &sc, i32 tri, float4 o, float4 d, float *u, f
 }
 
 // Slab test of both children of a node.  Box tests only decide what is skipped, never which
-// triangle is hit (boxes are expanded by 1e-3, far above rounding), so they use fused
+// triangle is hit (boxes are expanded past their rounding, bvh_margin.hpp), so they use fused
 // multiply-add t = box*inv - origin*inv: one instruction per plane.
 PHX_DI void box2(const float4 &a, const float4 &b, const float4 &c, float ix, float iy, float iz, float oix, float oiy,
                  float oiz, float t_min, float t_max, float *tl, float *tr, bool *hl, bool *hr) {
@@ -215,9 +216,10 @@ PHX_DI float qbox(u32 nxw, u32 fxw, u32 nyw, u32 fyw, u32 nzw, u32 fzw, int k, f
 // visited most of the tree — 62,533 steps for one photon of the 1920x1080 atrium workload emitted
 // straight down, direction (0, 0, -1), from its point light: 26-40 ms added to about one round in
 // ten.  With 1e30 a slab's distances are (plane - oc) * 1e30 up to a rounding
-// of |oc| * 2^-24 * 1e30, so their signs are exact for every plane farther than 6e-4 from oc, as
-// is every plane of a box holding a triangle the ray can hit (triangle boxes are widened by 1e-3
-// and the ray's coordinate must lie within the triangle's range).  A box that oc lies outside of
+// of |oc| * 2^-24 * 1e30, so their signs are exact for every plane farther than |oc| * 2^-24 from oc, as
+// is every plane of a box holding a triangle the ray can hit (such a box is widened by at least 128 * 2^-24
+// of the largest coordinate a ray starts from, or by 1e-3, and the ray's coordinate must lie within
+// the triangle's range).  A box that oc lies outside of
 // gets two distances of one sign, at least ~1e27 in magnitude, and is pruned.  NaN and finite
 // inverses are unchanged.
 PHX_DI float slab_inv(float dc, float oc) {

@@ -30,6 +30,7 @@
 //                 d log Φ_k/dθ (the bounces before the store and 1/L of its light)
 // Gradients are summed per block in shared memory (float) and then into doubles.
 #include "dev_shading.cuh"
+#include "gather_walk.cuh"
 #include "kernels.hpp"
 
 #include <algorithm>
@@ -613,63 +614,69 @@ __global__ void __launch_bounds__(128) k_emit_adj(LaunchCtx lc, AdjBufs ab) {
 }
 
 // ---- gather adjoint (gather_flux.cl:5-78, photon_hash.h:56-103) --------------------------------
-__global__ void __launch_bounds__(128) k_gather_adj(LaunchCtx lc, GatherBufs g, AdjBufs ab) {
-    u32 gpix = blockIdx.x * blockDim.x + threadIdx.x;
-    if (gpix >= lc.total_pixels)
-        return;
-    if (g.order) // any round's order will do: it only decides which pixels share a warp
-        gpix = __ldg(&g.order[gpix]);
+// Bound by the photon records' latency and, before the walk of the forward gather was shared, by the few lanes
+// that ran a pair's weight, loads and reduction while the others waited: with the queue they run together.
+// A round's 16-byte reductions stay, one a pair.  One-round step of the 512 x 512 atrium 5.38 -> 4.79 ms,
+// two-round step of a 97 x 65 caustic box 2.69 -> 2.48.  8 blocks an SM and two pairs in flight: a pair holds
+// a record index more than the forward gather's.
+constexpr u32 GA_BATCH = 2;
+__global__ void __launch_bounds__(128, 8) k_gather_adj(LaunchCtx lc, GatherBufs g, AdjBufs ab) {
+    __shared__ u32 q_k[GQ_CAP][128];
+    __shared__ float q_d[GQ_CAP][128];
+    const u32 tid = threadIdx.x;
+    u32 gpix = blockIdx.x * blockDim.x + tid;
     const SceneDesc &sc = lc.scenes[0];
-    const float4 ge = g.hp_emission[gpix];
-    const float4 a = ab.g_img[gpix] * ab.kscale[gpix];
-    if (ge.w == 0.0f || (a.x == 0.0f && a.y == 0.0f && a.z == 0.0f)) {
-        ab.gT[gpix] = zero4();
-        ab.gA[gpix] = zero4();
-        return;
-    }
-    const GridDev grid = sc.grid;
-    const float r_sq = ab.r2[gpix];
-    const float4 pos = g.hp_pos[gpix];
-    const float4 nrm = g.hp_normal[gpix];
-    const float4 T = g.hp_throughput[gpix], A = g.hp_base_color[gpix];
-    const float4 pa = a * T * (A / PI); // dL/dΦ_k = w_k · pa
-    const float denom = 2.0f * r_sq;
-    const float qx = (pos.x - grid.ox) / grid.cx, qy = (pos.y - grid.oy) / grid.cy, qz = (pos.z - grid.oz) / grid.cz;
-    const u32 G = grid.g;
-    constexpr float M = 1.0f / 1024.0f;
-    float4 S = zero4();
-    const u32 *cs = g.cell_start + sc.cell_base;
-    for (u32 i = 0; i < 27; i++) {
-        float px = pos.x, py = pos.y, pz = pos.z;
-        px += (float)((i32)(i % 3) - 1) * grid.cx;
-        py += (float)((i32)((i / 3) % 3) - 1) * grid.cy;
-        pz += (float)((i32)((i / 9) % 3) - 1) * grid.cz;
-        const u32 hsh = get_hash(px, py, pz, grid);
-        if (hsh == 0)
-            continue;
-        const u32 hz = (hsh - 1) % G, hy = ((hsh - 1) / G) % G, hx = (hsh - 1) / (G * G);
-        const float gx = fmaxf(fmaxf(((float)hx - M) - qx, qx - ((float)hx + (1.0f + M))), 0.0f) * grid.cx;
-        const float gy = fmaxf(fmaxf(((float)hy - M) - qy, qy - ((float)hy + (1.0f + M))), 0.0f) * grid.cy;
-        const float gz = fmaxf(fmaxf(((float)hz - M) - qz, qz - ((float)hz + (1.0f + M))), 0.0f) * grid.cz;
-        if ((gx * gx + gy * gy) + gz * gz > r_sq)
-            continue;
-        const u32 end = min(__ldg(&cs[hsh + 1]), g.n_cap);
-        for (u32 k = min(__ldg(&cs[hsh]), g.n_cap); k < end; k++) {
-            const float4 p = __ldg(&g.s_posdir[k]);
-            const float dx = pos.x - p.x, dy = pos.y - p.y, dz = pos.z - p.z, dw = pos.w - 0.0f;
-            const float dsq = ((dx * dx + dy * dy) + dz * dz) + dw * dw;
-            if (!(dsq < r_sq))
-                continue;
-            if (dot(__ldg(&g.s_dir[k]), nrm) > 0.0f) // decode_oct(p.w)
-                continue;
-            const float w = GAUSS_ALPHA * (1.0f - (1.0f - pm_expf((-GAUSS_BETA) * dsq / denom)) / GAUSS_DENOM);
-            const u32 c = __ldg(&ab.perm[k]);
-            S += w * __ldg(&ab.ph_pow[c]);
-            atomicAdd(&ab.gphi[c], f4(w * pa.x, w * pa.y, w * pa.z, 0.0f)); // one 16-byte reduction (1.09 -> 0.74 ms with the order)
+    bool gathering = false;
+    float4 a = zero4(), pos = zero4(), nrm = zero4(), pa = zero4(), S = zero4();
+    float r_sq = 0.0f;
+    NearCells nc;
+    if (gpix < lc.total_pixels) {
+        if (g.order) // any round's order will do: it only decides which pixels share a warp
+            gpix = __ldg(&g.order[gpix]);
+        a = ab.g_img[gpix] * ab.kscale[gpix];
+        gathering = !(g.hp_emission[gpix].w == 0.0f || (a.x == 0.0f && a.y == 0.0f && a.z == 0.0f));
+        if (!gathering) {
+            ab.gT[gpix] = zero4();
+            ab.gA[gpix] = zero4();
         }
     }
-    ab.gT[gpix] = a * (A / PI) * S;
-    ab.gA[gpix] = a * (T / PI) * S;
+    if (gathering) {
+        r_sq = ab.r2[gpix];
+        pos = g.hp_pos[gpix];
+        nrm = g.hp_normal[gpix];
+        pa = a * g.hp_throughput[gpix] * (g.hp_base_color[gpix] / PI); // dL/dΦ_k = w_k · pa
+        nc = near_cells(pos, r_sq, sc.grid);
+    }
+    const KernelWeight weight(r_sq);
+    walk_photons(g, g.cell_start + sc.cell_base, sc.grid.g, nc, pos, r_sq, q_k, q_d, tid, [&](u32 cnt) {
+        for (u32 e = 0; __any_sync(0xffffffffu, e < cnt); e += GA_BATCH) {
+            if (e >= cnt)
+                continue;
+            float4 pd[GA_BATCH], pw[GA_BATCH];
+            u32 c[GA_BATCH];
+#pragma unroll
+            for (u32 u = 0; u < GA_BATCH; u++) {
+                const u32 k = q_k[min(e + u, cnt - 1u)][tid];
+                c[u] = __ldg(&ab.perm[k]);
+                pd[u] = __ldg(&g.s_dir[k]); // decode_oct(p.w)
+            }
+#pragma unroll
+            for (u32 u = 0; u < GA_BATCH; u++)
+                pw[u] = __ldg(&ab.ph_pow[c[u]]);
+#pragma unroll
+            for (u32 u = 0; u < GA_BATCH; u++) {
+                if (e + u < cnt && !(dot(pd[u], nrm) > 0.0f)) {
+                    const float w = weight(q_d[e + u][tid]);
+                    S += w * pw[u];
+                    atomicAdd(&ab.gphi[c[u]], f4(w * pa.x, w * pa.y, w * pa.z, 0.0f)); // one 16-byte reduction
+                }
+            }
+        }
+    });
+    if (!gathering)
+        return;
+    ab.gT[gpix] = a * (g.hp_base_color[gpix] / PI) * S;
+    ab.gA[gpix] = a * (g.hp_throughput[gpix] / PI) * S;
 }
 
 // ---- small kernels -------------------------------------------------------------------------------

@@ -8,42 +8,9 @@
 // reference's cell order and each cell in sorted (= canonical) order, in one thread with no float
 // atomics, so the sum is deterministic and equal to the reference's sequential sum.  cell_end is
 // not materialised: the cells are contiguous, so end(h) = start(h+1).
-#include "kernels.hpp"
+#include "gather_walk.cuh"
 
 namespace phx {
-
-// x / y from r = 1 / y, for the many x of one y.  Markstein's theorem ("Computation of elementary functions on
-// the IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990): if r is 1/y rounded to nearest and q
-// within one ulp of x/y, then q + (x - q y) r, each step one fused multiply-add, is x/y rounded to
-// nearest.  x r alone is within 1.5 ulp, so a first step brings it within one and the second is exact.
-// Needs x/y, x and x 2^-24 in the normal range.
-PHX_DI float div_known(float x, float y, float r) {
-    float q = x * r;
-    q = __fmaf_rn(__fmaf_rn(-q, y, x), r, q);
-    return __fmaf_rn(__fmaf_rn(-q, y, x), r, q);
-}
-// x / GAUSS_DENOM for x = 0 or in [2^-30, 1.5]: one step is enough (every such x was checked).
-PHX_DI float div_gauss(float x) {
-    constexpr float r = 1.0f / GAUSS_DENOM;
-    const float q = x * r;
-    return __fmaf_rn(__fmaf_rn(-q, GAUSS_DENOM, x), r, q);
-}
-
-// pm_expf for t in [-1, 0]: its operations without its range checks.
-PHX_DI float exp_unit(float t) {
-    const float kf = floorf(t * PM_LOG2E + 0.5f); // 0 or -1
-    float r = t - kf * PM_LN2_HI;
-    r = r - kf * PM_LN2_LO;
-    float p = 1.984126984126984e-04f;
-    p = p * r + 1.388888888888889e-03f;
-    p = p * r + 8.333333333333333e-03f;
-    p = p * r + 4.1666666666666664e-02f;
-    p = p * r + 1.6666666666666666e-01f;
-    p = p * r + 0.5f;
-    p = p * r + 1.0f;
-    p = p * r + 1.0f;
-    return kf < 0.0f ? p * 0.5f : p;
-}
 
 // One pixel per thread, in two alternating phases.  The lanes of a warp walk their cells' photons four at a
 // time and only queue those inside the radius (a few instructions each, no branch to a rare long
@@ -55,7 +22,7 @@ PHX_DI float exp_unit(float t) {
 // workload), 3.88 -> 1.82 (atrium), 0.40 -> 0.25 (512 x 512 Cornell).  16 queue places, 8 blocks per SM
 // and batches of 3 measured best of 12..32, 6..12 and 1..4 (more blocks spill, smaller queues empty
 // while most lanes hold few).
-constexpr u32 GQ_CAP = 16, GQ_AHEAD = 4, GQ_BATCH = 3;
+constexpr u32 GQ_BATCH = 3;
 __global__ void __launch_bounds__(128, 8) k_gather(LaunchCtx lc, GatherBufs g) {
     __shared__ u32 q_k[GQ_CAP][128];
     __shared__ float q_d[GQ_CAP][128];
@@ -65,7 +32,7 @@ __global__ void __launch_bounds__(128, 8) k_gather(LaunchCtx lc, GatherBufs g) {
     bool gathering = false;
     float4 pos = zero4(), nrm = zero4(), nf = zero4();
     float r_sq = 0.0f, found = 0.0f;
-    u32 wx = 0, wy = 0, wz = 0, near = 0; // cell coordinates per axis, and the cells within the radius
+    NearCells nc;
     const SceneDesc *scp = lc.scenes;
     if (gpix < lc.total_pixels) {
         if (g.order)
@@ -93,8 +60,6 @@ __global__ void __launch_bounds__(128, 8) k_gather(LaunchCtx lc, GatherBufs g) {
     }
     const SceneDesc &sc = *scp;
     const GridDev grid = sc.grid;
-    const u32 *cs = g.cell_start + sc.cell_base;
-    const u32 G = grid.g;
     if (gathering) {
         r_sq = g.flux[gpix].w;
         if (r_sq < EPS) {
@@ -103,60 +68,10 @@ __global__ void __launch_bounds__(128, 8) k_gather(LaunchCtx lc, GatherBufs g) {
         }
         pos = g.hp_pos[gpix];
         nrm = g.hp_normal[gpix];
-        // The 27 cells in the reference's order (photon_hash.h:65-82), each in sorted (canonical)
-        // photon order.  A cell whose box lies farther than the search radius from the hit point holds
-        // no photon with dsq < r_sq, so it adds nothing and is skipped; the box is widened by 1/1024
-        // of a cell on every side so that rounding in get_hash (which decides a photon's cell) and in
-        // this test can never skip a photon that would count.
-        // get_hash of a neighbour position works axis by axis, and an axis's coordinate only takes the
-        // three values pos + {-1, 0, 1} * cell: each axis's three cell coordinates are computed once,
-        // with the same operations get_hash applies, and packed one byte per offset; an axis's three
-        // squared distances decide the cells together (infinite outside the grid, which has at most 255
-        // cells per axis).
-        constexpr float M = 1.0f / 1024.0f;
-        const float gf = (float)G;
-        float d2[3][3];
-        auto axis_cells = [&](float p, float o, float c, float (&d)[3]) -> u32 {
-            const float q0 = (p - o) / c; // the hit point in cell units
-            u32 w = 0;
-#pragma unroll
-            for (int k = 0; k < 3; k++) {
-                float q = p;
-                q += (float)(k - 1) * c;
-                const float f = (q - o) / c;
-                const bool in = !(f < 0.0f || f >= gf);
-                const u32 ci = in ? (u32)f : 0u;
-                const float gap = fmaxf(fmaxf(((float)ci - M) - q0, q0 - ((float)ci + (1.0f + M))), 0.0f) * c;
-                d[k] = in ? gap * gap : __int_as_float(0x7f800000);
-                w |= ci << (8 * k);
-            }
-            return w;
-        };
-        wx = axis_cells(pos.x, grid.ox, grid.cx, d2[0]);
-        wy = axis_cells(pos.y, grid.oy, grid.cy, d2[1]);
-        wz = axis_cells(pos.z, grid.oz, grid.cz, d2[2]);
-#pragma unroll
-        for (u32 c = 0; c < 27; c++) {
-            const float dx = d2[0][c % 3], dy = d2[1][(c / 3) % 3], dz = d2[2][c / 9];
-            if (!((dx + dy) + dz > r_sq) && dx + dy + dz < __int_as_float(0x7f800000))
-                near |= 1u << c;
-        }
+        nc = near_cells(pos, r_sq, grid);
     }
-    const float denom = 2.0f * r_sq, dw = pos.w - 0.0f;
-    const float rdenom = 1.0f / denom;
-    const float dsq_min = denom > 1e-18f && denom < 1e18f ? 1e-30f : __int_as_float(0x7f800000);
-    // the photon range of the next cell of `near`
-    auto next_cell = [&](u32 *lo, u32 *hi) {
-        const u32 c = (u32)__ffs(near) - 1u, c3 = c / 3u;
-        near &= near - 1u;
-        const u32 hx = (wx >> (8u * (c - 3u * c3))) & 0xffu, hy = (wy >> (8u * (c3 % 3u))) & 0xffu,
-                  hz = (wz >> (8u * (c / 9u))) & 0xffu;
-        const u32 h = G * G * hx + G * hy + hz + 1; // get_hash's cell index
-        *lo = min(__ldg(&cs[h]), g.n_cap);
-        *hi = min(__ldg(&cs[h + 1]), g.n_cap);
-    };
-    u32 cnt = 0;
-    auto flush = [&]() {
+    const KernelWeight weight(r_sq);
+    walk_photons(g, g.cell_start + sc.cell_base, grid.g, nc, pos, r_sq, q_k, q_d, tid, [&](u32 cnt) {
         for (u32 e = 0; __any_sync(FULL, e < cnt); e += GQ_BATCH) {
             if (e >= cnt)
                 continue;
@@ -170,10 +85,7 @@ __global__ void __launch_bounds__(128, 8) k_gather(LaunchCtx lc, GatherBufs g) {
 #pragma unroll
             for (u32 u = 0; u < GQ_BATCH; u++) {
                 if (e + u < cnt && !((pd[u].x * nrm.x + pd[u].y * nrm.y) + pd[u].z * nrm.z > 0.0f)) { // both w are 0
-                    const float dsq = q_d[e + u][tid];
-                    const float x = (-GAUSS_BETA) * dsq;
-                    const float t = dsq >= dsq_min ? div_known(x, denom, rdenom) : x / denom;
-                    const float w = GAUSS_ALPHA * (1.0f - div_gauss(1.0f - exp_unit(t)));
+                    const float w = weight(q_d[e + u][tid]);
                     nf.x += w * pw[u].x;
                     nf.y += w * pw[u].y;
                     nf.z += w * pw[u].z;
@@ -181,44 +93,7 @@ __global__ void __launch_bounds__(128, 8) k_gather(LaunchCtx lc, GatherBufs g) {
                 }
             }
         }
-        cnt = 0;
-    };
-    u32 k = 0, end = 0, n0 = 0, n1 = 0;
-    bool ahead = near != 0; // n0, n1: the range of the cell after the current one, loaded ahead
-    if (ahead)
-        next_cell(&n0, &n1);
-    for (;;) {
-        while (k >= end && ahead) { // the next cell with photons
-            k = n0;
-            end = n1;
-            ahead = near != 0;
-            if (ahead)
-                next_cell(&n0, &n1);
-        }
-        __syncwarp();
-        if (!__any_sync(FULL, k < end))
-            break;
-        if (k < end) {
-            float4 p[GQ_AHEAD];
-#pragma unroll
-            for (u32 u = 0; u < GQ_AHEAD; u++)
-                p[u] = __ldg(&g.s_posdir[min(k + u, end - 1u)]);
-#pragma unroll
-            for (u32 u = 0; u < GQ_AHEAD; u++) {
-                const float dx = pos.x - p[u].x, dy = pos.y - p[u].y, dz = pos.z - p[u].z;
-                const float dsq = ((dx * dx + dy * dy) + dz * dz) + dw * dw;
-                if (dsq < r_sq && k + u < end) {
-                    q_k[cnt][tid] = k + u;
-                    q_d[cnt][tid] = dsq;
-                    cnt++;
-                }
-            }
-            k += GQ_AHEAD;
-        }
-        if (__any_sync(FULL, cnt > GQ_CAP - GQ_AHEAD))
-            flush();
-    }
-    flush();
+    });
     if (!gathering)
         return;
     const float4 fso = g.flux[gpix];

@@ -504,7 +504,8 @@ PHX_API int phx_scan_noalloc(const uint32_t *in, uint32_t *out, uint32_t n, uint
  *              the reference raises for k > 2: PHX_E_INVALID);
  *   weighted:  sum of value * weights[(yy - y + k) * (2k + 1) + (xx - x + k)]; `weights` holds
  *              (2k+1)^2 floats (gaussian_filter_gpu passes the normalised Gaussian).
- * k <= 32.  Synchronous on a stream of its own on the current device.  kernel_ms, if not NULL,
+ * k <= 32.  Synchronous on a stream of its own on the current device.  `out` may overlap `in` (an
+ * in-place call): it is written after the image has been read.  kernel_ms, if not NULL,
  * receives the filter kernel's CUDA-event time (copies excluded). */
 PHX_API int phx_mean_filter(const int32_t *in, float *out, uint32_t width, uint32_t height, uint32_t k,
                             float *kernel_ms);

@@ -76,8 +76,8 @@ template <> struct Pow2<1> {
 // The image is staged as float for the sums (each value converted once: the same value the
 // kernels' per-use (float) conversion gives) and as int for the median.  The three channels are
 // summed together; each channel's additions keep the kernels' order.
-// IN: int, or unsigned char (an 8-bit image: the same values in a quarter of the bytes).  OUT: float, or
-// double (the float result, widened where it is written).
+// IN: int, or unsigned char (an 8-bit image: the same values in a quarter of the bytes; with double only).
+// OUT: float, or double (the float result, widened where it is written).
 template <int MODE, bool TILED, int MK, class IN, class OUT>
 __global__ void __launch_bounds__(BX *BY) k_filter(const IN *__restrict__ in, OUT *__restrict__ out,
                                                    const float *__restrict__ weights, int width, int height, int k) {
@@ -247,6 +247,10 @@ int denoise_filter(int mode, const void *in, bool in_u8, void *out, bool out_f64
         msg = "window radius k must be <= 32";
         return 1;
     }
+    if (in_u8 && !out_f64) {
+        msg = "8-bit images have a float64 result";
+        return 1;
+    }
     const size_t n = (size_t)width * height * 3, nw = (size_t)(2 * k + 1) * (2 * k + 1);
     const size_t in_bytes = n * (in_u8 ? 1 : 4), out_bytes = n * (out_f64 ? 8 : 4);
     cudaStream_t st = nullptr;
@@ -275,10 +279,8 @@ int denoise_filter(int mode, const void *in, bool in_u8, void *out, bool out_f64
     if (ok()) {
         const int w = (int)width, h = (int)height, kk = (int)k;
         auto go = [&](auto *i, auto *o) { launch_filter(mode, i, o, d_w, w, h, kk, st); };
-        if (in_u8 && out_f64)
+        if (in_u8)
             go((const unsigned char *)d_in, (double *)d_out);
-        else if (in_u8)
-            go((const unsigned char *)d_in, (float *)d_out);
         else if (out_f64)
             go((const int *)d_in, (double *)d_out);
         else

@@ -28,7 +28,8 @@
 //   k_nee_adj     the transmissive surfaces those samples' shadow rays crossed
 //   k_emit_adj    replays the photon path; at stored photon k, u = dL/dΦ_k ⊙ Φ_k times
 //                 d log Φ_k/dθ (the bounces before the store and 1/L of its light)
-// Gradients are summed per block in shared memory (float) and then into doubles.
+// Gradients are summed per block in shared memory (float) and then into doubles; with more parameters than a
+// block's shared memory holds, every term goes into a double by itself.
 #include "dev_shading.cuh"
 #include "gather_walk.cuh"
 #include "kernels.hpp"
@@ -38,23 +39,39 @@
 namespace phx {
 
 // ---- gradient accumulation ---------------------------------------------------------------------
-struct GradAcc {
-    float *sm;  // per-block partial sums (nullptr: straight to global)
+// S, the type that sums of terms are held in: float where a block has partial sums in shared memory
+// (AdjBufs::block_sums), double where each sum goes straight to the global doubles, whose precision a float
+// in between would lose.
+template <class S> struct Sum3 {
+    S x = 0, y = 0, z = 0;
+    Sum3() = default;
+    PHX_DI explicit Sum3(float4 v, float s = 1.0f) : x(v.x * (S)s), y(v.y * (S)s), z(v.z * (S)s) {}
+    PHX_DI Sum3 &operator+=(const Sum3 &o) {
+        x += o.x;
+        y += o.y;
+        z += o.z;
+        return *this;
+    }
+    PHX_DI bool any() const { return x != 0 || y != 0 || z != 0; }
+};
+
+template <class S> struct GradAcc {
+    float *sm; // per-block partial sums (S = float)
     double *gl;
-    PHX_DI void add(u32 i, float v) const {
-        if (v == 0.0f)
+    PHX_DI void add(u32 i, S v) const {
+        if (v == 0)
             return;
-        if (sm)
+        if constexpr (sizeof(S) == 4)
             atomicAdd(&sm[i], v);
         else
-            atomicAdd(&gl[i], (double)v);
+            atomicAdd(&gl[i], v);
     }
     // Four consecutive entries at once.  The lanes that add to the same entries (most of a warp: few
     // materials hold most hits) sum their values by shuffles first: a shared-memory float addition is a
-    // compare-and-swap loop, which 32 lanes on one address run 32 times.
-    PHX_DI void add4(u32 o, float a, float b, float c, float d) const {
+    // compare-and-swap loop, which 32 lanes on one address run 32 times, and a global one serialises as well.
+    PHX_DI void add4(u32 o, S a, S b, S c, S d) const {
         const u32 peers = __match_any_sync(__activemask(), o);
-        float s0 = 0.0f, s1 = 0.0f, s2 = 0.0f, s3 = 0.0f;
+        S s0 = 0, s1 = 0, s2 = 0, s3 = 0;
         for (u32 m = peers; m; m &= m - 1u) {
             const int src = __ffs(m) - 1;
             s0 += __shfl_sync(peers, a, src);
@@ -69,25 +86,25 @@ struct GradAcc {
             add(o + 3, s3);
         }
     }
-    PHX_DI void add3(u32 o, float a, float b, float c) const { add4(o, a, b, c, 0.0f); }
+    // z ⊙ v to three entries
+    PHX_DI void add3(u32 o, const Sum3<S> &z, float4 v) const { add4(o, z.x * v.x, z.y * v.y, z.z * v.z, 0); }
 };
 
-PHX_DI GradAcc grad_begin(const AdjBufs &ab, float *smem) {
-    GradAcc g{ab.block_sums ? smem : nullptr, ab.grad};
-    if (g.sm) {
+template <class S> PHX_DI GradAcc<S> grad_begin(const AdjBufs &ab, float *smem) {
+    if constexpr (sizeof(S) == 4) {
         for (u32 i = threadIdx.x; i < ab.n_params; i += blockDim.x)
-            g.sm[i] = 0.0f;
+            smem[i] = 0.0f;
         __syncthreads();
     }
-    return g;
+    return GradAcc<S>{smem, ab.grad};
 }
-PHX_DI void grad_end(const AdjBufs &ab, const GradAcc &g) {
-    if (!g.sm)
-        return;
-    __syncthreads();
-    for (u32 i = threadIdx.x; i < ab.n_params; i += blockDim.x)
-        if (g.sm[i] != 0.0f)
-            atomicAdd(&ab.grad[i], (double)g.sm[i]);
+template <class S> PHX_DI void grad_end(const AdjBufs &ab, const GradAcc<S> &g) {
+    if constexpr (sizeof(S) == 4) {
+        __syncthreads();
+        for (u32 i = threadIdx.x; i < ab.n_params; i += blockDim.x)
+            if (g.sm[i] != 0.0f)
+                atomicAdd(&ab.grad[i], (double)g.sm[i]);
+    }
 }
 
 // ---- log-derivatives of the weights ------------------------------------------------------------
@@ -147,10 +164,10 @@ PHX_DI BounceRec bounce_dlog(const BsdfSample &bs, float4 h, float4 view, float4
 
 // Adds Σ_c z_c · d log W_i,c/dθ for every recorded bounce i (z = u ⊙ X of a term X that carries
 // the product of those bounce weights).
-PHX_DI void add_prefix(const GradAcc &acc, const BounceRec *br, u32 nb, float4 z) {
-    if (z.x == 0.0f && z.y == 0.0f && z.z == 0.0f)
+template <class S> PHX_DI void add_prefix(const GradAcc<S> &acc, const BounceRec *br, u32 nb, const Sum3<S> &z) {
+    if (!z.any())
         return;
-    const float zs = z.x + z.y + z.z;
+    const S zs = z.x + z.y + z.z;
     for (u32 i = 0; i < nb; i++) {
         acc.add4(4 * br[i].mat, z.x * br[i].db0, z.y * br[i].db1, z.z * br[i].db2, zs * br[i].dr);
     }
@@ -246,15 +263,13 @@ PHX_DI float4 nee_specular_adj(Rng *rng, const SceneDesc &sc, float4 pos, float4
 }
 
 // per-sample derivatives of a NEE term z = u ⊙ X: its light and its transmissive occluders
-PHX_DI void add_nee_common(const SceneDesc &sc, const AdjBufs &ab, const GradAcc &acc, const NeeRec &nr, float4 z) {
-    if (sc.n_lights > 0) {
-        const float4 il = inv_nonzero(f4(sc.lights[nr.light].power));
-        acc.add3(4 * ab.n_mat + 3 * nr.light, z.x * il.x, z.y * il.y, z.z * il.z);
-    }
-    for (u32 i = 0; i < nr.n_occ; i++) {
-        const float4 imb = inv_nonzero(f4(sc.materials[nr.occ[i]].base_color));
-        acc.add3(4 * nr.occ[i], z.x * imb.x, z.y * imb.y, z.z * imb.z);
-    }
+template <class S>
+PHX_DI void add_nee_common(const SceneDesc &sc, const AdjBufs &ab, const GradAcc<S> &acc, const NeeRec &nr,
+                           const Sum3<S> &z) {
+    if (sc.n_lights > 0)
+        acc.add3(4 * ab.n_mat + 3 * nr.light, z, inv_nonzero(f4(sc.lights[nr.light].power)));
+    for (u32 i = 0; i < nr.n_occ; i++)
+        acc.add3(4 * nr.occ[i], z, inv_nonzero(f4(sc.materials[nr.occ[i]].base_color)));
 }
 
 // ---- camera paths (trace_rays.cl:14-169) -------------------------------------------------------
@@ -265,9 +280,9 @@ PHX_DI void add_nee_common(const SceneDesc &sc, const AdjBufs &ab, const GradAcc
 // gT.  Otherwise (the one-thread camera kernel, or a specular event that found no free slots) the
 // samples are traced here, one after another: 6.2 ms for 512 x 512 pixels of the atrium at 16 samples,
 // against 0.72 ms recorded; 1.45 against 0.29 + 0.06 (k_nee_adj) for 97 x 65 pixels through glass at 8.
-template <bool REC>
-PHX_DI void trace_adj_pixel(const SceneDesc &sc, u32 seed, u32 tid, u32 gpix, const AdjBufs &ab, const GradAcc &acc,
-                            u32 *overflow) {
+template <bool REC, class S>
+PHX_DI void trace_adj_pixel(const SceneDesc &sc, u32 seed, u32 tid, u32 gpix, const AdjBufs &ab,
+                            const GradAcc<S> &acc, u32 *overflow) {
     const float4 ur = ab.g_img[gpix] * ab.inv_rounds; // dL / d(this round's radiance increment)
     const float4 uT = ab.gT[gpix], uA = ab.gA[gpix];
     if (ur.x == 0.0f && ur.y == 0.0f && ur.z == 0.0f && uT.x == 0.0f && uT.y == 0.0f && uT.z == 0.0f &&
@@ -295,7 +310,7 @@ PHX_DI void trace_adj_pixel(const SceneDesc &sc, u32 seed, u32 tid, u32 gpix, co
         bool hit = intersect(sc, origin, dir, EPS, INF, &h, overflow);
         if (!hit) {
             if (sc.has_env)
-                add_prefix(acc, br, nb, ur * throughput * sample_envmap(sc, dir));
+                add_prefix(acc, br, nb, Sum3<S>(ur * throughput * sample_envmap(sc, dir)));
             break;
         }
         const phx_material mat = sc.materials[tri_mat(sc, h.tri)];
@@ -307,7 +322,7 @@ PHX_DI void trace_adj_pixel(const SceneDesc &sc, u32 seed, u32 tid, u32 gpix, co
         if (mat.norm_index != NO_TEXTURE)
             hit_frame(sc, h, sh, &tangent, &bitangent);
         ShadingContext ctx = evaluate_material(sc, mat, sh.mat_index, sh.uvx, sh.uvy, sh.normal, tangent, bitangent);
-        add_prefix(acc, br, nb, ur * throughput * ctx.emissive);
+        add_prefix(acc, br, nb, Sum3<S>(ur * throughput * ctx.emissive));
         float4 view = -dir;
         float4 hm; // the microfacet normal
         BsdfSample bs = sample_bsdf_h(&rng, ctx, ctx.shading_normal, sh.normal, view, &ior, sh.front_face, &hm);
@@ -316,14 +331,17 @@ PHX_DI void trace_adj_pixel(const SceneDesc &sc, u32 seed, u32 tid, u32 gpix, co
         if (bs.event == BSDF_DIFFUSE) {
             // direct = T·occlusion·mean_s NEE_s, NEE_s = L_s·base/π·trans_s
             const float4 w = ur * throughput * (ctx.occlusion * inv_ds);
-            float4 zsum = zero4();
+            Sum3<S> zsum;
             if constexpr (REC) {
-                zsum = ur * ab.tr.direct[gpix];
+                const float4 *val = ab.tr.nee_val + sc.nee_base + (size_t)(gpix - sc.pixel_base) * sc.direct_samples;
+                if constexpr (sizeof(S) == 4)
+                    zsum = Sum3<S>(ur * ab.tr.direct[gpix]); // the pass's own float mean of the samples
+                else
+                    for (u32 d = 0; d < sc.direct_samples; d++)
+                        zsum += Sum3<S>(w * val[d]);
                 if (sc.n_lights == 1) {
-                    const float4 il = inv_nonzero(f4(sc.lights[0].power));
-                    acc.add3(4 * ab.n_mat, zsum.x * il.x, zsum.y * il.y, zsum.z * il.z);
+                    acc.add3(4 * ab.n_mat, zsum, inv_nonzero(f4(sc.lights[0].power)));
                 } else {
-                    const float4 *val = ab.tr.nee_val + sc.nee_base + (size_t)(gpix - sc.pixel_base) * sc.direct_samples;
                     for (u32 d = 0; d < sc.direct_samples; d++) { // which light each sample chose
                         NeeRec nr;
                         nr.n_occ = 0;
@@ -334,8 +352,8 @@ PHX_DI void trace_adj_pixel(const SceneDesc &sc, u32 seed, u32 tid, u32 gpix, co
                         } else {
                             rng = rng_advance(rng, sc.light_draws);
                         }
-                        const float4 z = w * val[d];
-                        if (z.x != 0.0f || z.y != 0.0f || z.z != 0.0f)
+                        const Sum3<S> z(w * val[d]);
+                        if (z.any())
                             add_nee_common(sc, ab, acc, nr, z);
                     }
                 }
@@ -345,16 +363,18 @@ PHX_DI void trace_adj_pixel(const SceneDesc &sc, u32 seed, u32 tid, u32 gpix, co
                     NeeRec nr;
                     float4 v =
                         nee_diffuse_adj(&rng, sc, sh.position, ctx.shading_normal, ctx.base_color, overflow, &nr);
-                    const float4 z = w * v;
-                    if (z.x == 0.0f && z.y == 0.0f && z.z == 0.0f)
+                    const Sum3<S> z(w * v);
+                    if (!z.any())
                         continue;
                     zsum += z;
                     add_nee_common(sc, ab, acc, nr, z);
                 }
             }
-            add_prefix(acc, br, nb, zsum + uT * throughput); // direct light, and the hit point's throughput
-            const float4 b = ctx.base_color;                 // the hit point's base colour (mb × texture)
-            acc.add3(mo, (zsum.x + uA.x * b.x) * imb.x, (zsum.y + uA.y * b.y) * imb.y, (zsum.z + uA.z * b.z) * imb.z);
+            Sum3<S> zp = zsum; // direct light, and the hit point's throughput
+            zp += Sum3<S>(uT * throughput);
+            add_prefix(acc, br, nb, zp);
+            zsum += Sum3<S>(uA * ctx.base_color); // the hit point's base colour (mb × texture)
+            acc.add3(mo, zsum, imb);
             break;
         }
         if (bs.event == BSDF_METALLIC || bs.event == BSDF_FRESNEL) {
@@ -366,15 +386,18 @@ PHX_DI void trace_adj_pixel(const SceneDesc &sc, u32 seed, u32 tid, u32 gpix, co
             }
             const float dadr = dalpha_drough(ctx.roughness, mat.roughness);
             const float4 w = ur * throughput * inv_ds;
-            float4 zsum = zero4(), gb = zero4(); // gb: d/d base colour (metal), d/d roughness
+            Sum3<S> zsum, gb; // gb, gr: d/d base colour (metal), d/d roughness
+            S gr = 0;
             u32 slots = DEF_KNOWN;
             if constexpr (REC) // the next event of the pixel's list (events past its slots are not in it)
                 while (at < n_list && slots == DEF_KNOWN)
                     slots = ab.tr.def_tag[(size_t)gpix * DEF_MAX + at++];
-            auto add_sample = [&](const NeeRec &nr, float4 z) {
+            auto add_sample = [&](const NeeRec &nr, const Sum3<S> &z) {
+                if (!z.any())
+                    return;
                 zsum += z;
                 add_nee_common(sc, ab, acc, nr, z);
-                gb.w += (z.x + z.y + z.z) * nr.dlog_a * dadr;
+                gr += (z.x + z.y + z.z) * nr.dlog_a * dadr;
                 if (bs.event == BSDF_METALLIC) { // f0 = base = mb × texture
                     const float4 b = ctx.base_color;
                     gb.x += z.x * nr.dlog_f0.x * b.x * imb.x;
@@ -388,26 +411,21 @@ PHX_DI void trace_adj_pixel(const SceneDesc &sc, u32 seed, u32 tid, u32 gpix, co
                 for (u32 d = 0; d < sc.direct_samples; d += same) {
                     NeeRec nr;
                     const Rng before = rng;
-                    const float4 known = ab.tr.spec_val[slots + d] * (float)same;
                     const float4 v = nee_specular_adj<true>(&rng, sc, sh.position, ctx.shading_normal, view, f0,
-                                                            ctx.roughness, overflow, &nr, known);
+                                                            ctx.roughness, overflow, &nr, ab.tr.spec_val[slots + d]);
                     if (same > 1 && rng.state != before.state)
                         rng = rng_advance(before, same * sc.light_draws);
-                    const float4 z = w * v;
-                    if (z.x != 0.0f || z.y != 0.0f || z.z != 0.0f)
-                        add_sample(nr, z);
+                    add_sample(nr, Sum3<S>(w * v, (float)same));
                 }
             } else {
                 for (u32 d = 0; d < sc.direct_samples; d++) {
                     NeeRec nr;
                     float4 v = nee_specular_adj<false>(&rng, sc, sh.position, ctx.shading_normal, view, f0,
                                                        ctx.roughness, overflow, &nr, zero4());
-                    const float4 z = w * v;
-                    if (z.x != 0.0f || z.y != 0.0f || z.z != 0.0f)
-                        add_sample(nr, z);
+                    add_sample(nr, Sum3<S>(w * v));
                 }
             }
-            acc.add4(mo, gb.x, gb.y, gb.z, gb.w);
+            acc.add4(mo, gb.x, gb.y, gb.z, gr);
             add_prefix(acc, br, nb, zsum);
         }
         br[nb++] = bounce_dlog(bs, hm, view, ctx.shading_normal, ctx, mat, sh.mat_index);
@@ -425,15 +443,15 @@ PHX_DI void trace_adj_pixel(const SceneDesc &sc, u32 seed, u32 tid, u32 gpix, co
     }
 }
 
-template <bool REC>
+template <bool REC, class S>
 __global__ void __launch_bounds__(128) k_trace_adj(LaunchCtx lc, AdjBufs ab) {
     extern __shared__ float s_grad[];
-    const GradAcc acc = grad_begin(ab, s_grad);
+    const GradAcc<S> acc = grad_begin<S>(ab, s_grad);
     u32 gid = blockIdx.x * blockDim.x + threadIdx.x;
     if (gid < lc.total_pixels) {
         const SceneDesc &sc = lc.scenes[0];
         u32 ovf = 0;
-        trace_adj_pixel<REC>(sc, __ldg(&lc.seeds[0]), gid, gid, ab, acc, &ovf);
+        trace_adj_pixel<REC, S>(sc, __ldg(&lc.seeds[0]), gid, gid, ab, acc, &ovf);
         if (ovf)
             atomicAdd(lc.overflow, ovf);
     }
@@ -443,28 +461,25 @@ __global__ void __launch_bounds__(128) k_trace_adj(LaunchCtx lc, AdjBufs ab) {
 // Occluders of the recorded NEE samples (scenes with transmissive materials): one thread per sample slot,
 // the diffuse hit points' first, then the specular events'.  A sample that contributes is drawn again
 // as the shadow pass drew it and its ray traced once more for the surfaces it crossed.
-__global__ void __launch_bounds__(128) k_nee_adj(LaunchCtx lc, AdjBufs ab, u32 nee_blocks) {
+template <class S> __global__ void __launch_bounds__(128) k_nee_adj(LaunchCtx lc, AdjBufs ab, u32 nee_blocks) {
     extern __shared__ float s_grad[];
-    const GradAcc acc = grad_begin(ab, s_grad);
+    const GradAcc<S> acc = grad_begin<S>(ab, s_grad);
     const SceneDesc &sc = lc.scenes[0];
     const TraceOut &out = ab.tr;
     const u32 ds = sc.direct_samples, same = ab.same_samples ? ds : 1u;
     u32 ovf = 0;
-    auto crossed = [&](float4 org, float4 dir, float dist, float4 z) {
+    auto crossed = [&](float4 org, float4 dir, float dist, const Sum3<S> &z) {
         NeeRec nr;
         shadow_tr_rec(sc, org, dir, dist, &ovf, &nr);
-        for (u32 i = 0; i < nr.n_occ; i++) {
-            const float4 imb = inv_nonzero(f4(sc.materials[nr.occ[i]].base_color));
-            acc.add3(4 * nr.occ[i], z.x * imb.x, z.y * imb.y, z.z * imb.z);
-        }
+        for (u32 i = 0; i < nr.n_occ; i++)
+            acc.add3(4 * nr.occ[i], z, inv_nonzero(f4(sc.materials[nr.occ[i]].base_color)));
     };
-    auto nonzero = [](float4 z) { return z.x != 0.0f || z.y != 0.0f || z.z != 0.0f; };
     if (blockIdx.x < nee_blocks) {
         const u32 t = (blockIdx.x * blockDim.x + threadIdx.x) * same;
         if (t < lc.total_nee && out.emission[t / ds].w == 1.0f) {
             const u32 gpix = t / ds;
-            const float4 z = ab.gT[gpix] * out.nee_val[t] * (float)same;
-            if (nonzero(z)) {
+            const Sum3<S> z(ab.gT[gpix] * out.nee_val[t], (float)same);
+            if (z.any()) {
                 if (sc.light_draws != LIGHT_DRAWS_VARY) {
                     Rng rng;
                     rng.state = out.stash_rng[gpix];
@@ -483,12 +498,13 @@ __global__ void __launch_bounds__(128) k_nee_adj(LaunchCtx lc, AdjBufs ab, u32 n
         for (u32 e = (blockIdx.x - nee_blocks) * blockDim.x + threadIdx.x; (u64)e * same < n; e += stride) {
             const u32 g = e * same, base = g / ds * ds; // events claim ds slots each
             const u32 gpix = out.spec_pix[g], listed = out.def_cnt[gpix] & 0xffu;
-            float4 z = zero4();
+            Sum3<S> z;
             for (u32 k = 0; k < listed; k++)
                 if (out.def_tag[(size_t)gpix * DEF_MAX + k] == base)
-                    z = ab.g_img[gpix] * ab.inv_rounds * out.def_val[(size_t)gpix * DEF_MAX + k] *
-                        (1.0f / (float)ds) * out.spec_val[g] * (float)same;
-            if (!nonzero(z))
+                    z = Sum3<S>(ab.g_img[gpix] * ab.inv_rounds * out.def_val[(size_t)gpix * DEF_MAX + k] *
+                                    (1.0f / (float)ds) * out.spec_val[g],
+                                (float)same);
+            if (!z.any())
                 continue;
             const float4 hdr = out.spec_ray[g];
             if (spec_drawn_in_shadow(sc)) {
@@ -511,7 +527,8 @@ __global__ void __launch_bounds__(128) k_nee_adj(LaunchCtx lc, AdjBufs ab, u32 n
 // ---- photon paths (emit_photons.cl:12-114) -----------------------------------------------------
 constexpr u32 MAX_PHOTON_BOUNCES = 32;
 
-PHX_DI void emit_adj_path(const SceneDesc &sc, u32 seed, u32 tid, const AdjBufs &ab, const GradAcc &acc,
+template <class S>
+PHX_DI void emit_adj_path(const SceneDesc &sc, u32 seed, u32 tid, const AdjBufs &ab, const GradAcc<S> &acc,
                           u32 *overflow) {
     u32 k = ab.offsets[tid];
     const u32 n_stored = ab.offsets[tid + 1] - k;
@@ -576,13 +593,13 @@ PHX_DI void emit_adj_path(const SceneDesc &sc, u32 seed, u32 tid, const AdjBufs 
     }
     // bounce i weighs every photon stored after it; the light weighs all of them: one sum per bounce, not
     // one per bounce and photon (atrium, 2^20 paths: 1.60 -> 1.06 ms with the shuffled sums)
-    float4 z = zero4();
+    Sum3<S> z;
     for (u32 i = nb; i-- > 0;) {
-        if (i + 1 < nb && (z.x != 0.0f || z.y != 0.0f || z.z != 0.0f))
+        if (i + 1 < nb && z.any())
             acc.add4(4 * br[i].mat, z.x * br[i].db0, z.y * br[i].db1, z.z * br[i].db2, (z.x + z.y + z.z) * br[i].dr);
-        z += stored[i];
+        z += Sum3<S>(stored[i]);
     }
-    acc.add3(lo, z.x * il.x, z.y * il.y, z.z * il.z);
+    acc.add3(lo, z, il);
 }
 
 // The paths that stored a photon (one in six of the atrium's), so that every lane of k_emit_adj has one to
@@ -599,9 +616,9 @@ __global__ void __launch_bounds__(256) k_adj_paths(LaunchCtx lc, AdjBufs ab) {
         ab.paths[base + __popc(m & ((1u << lane) - 1u))] = gid;
 }
 
-__global__ void __launch_bounds__(128) k_emit_adj(LaunchCtx lc, AdjBufs ab) {
+template <class S> __global__ void __launch_bounds__(128) k_emit_adj(LaunchCtx lc, AdjBufs ab) {
     extern __shared__ float s_grad[];
-    const GradAcc acc = grad_begin(ab, s_grad);
+    const GradAcc<S> acc = grad_begin<S>(ab, s_grad);
     const u32 i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < *ab.n_paths) {
         const SceneDesc &sc = lc.scenes[0];
@@ -734,26 +751,36 @@ __global__ void __launch_bounds__(256) k_adj_image(const float4 *flux, const flo
 
 static size_t grad_smem(const AdjBufs &ab) { return ab.block_sums ? 4 * (size_t)ab.n_params : 0; }
 
+template <class S> static void launch_trace_adj_s(const LaunchCtx &lc, const AdjBufs &ab, cudaStream_t st) {
+    const u32 grid = (lc.total_pixels + 127) / 128;
+    if (!ab.tr.def_cnt) {
+        k_trace_adj<false, S><<<grid, 128, grad_smem(ab), st>>>(lc, ab);
+        return;
+    }
+    k_trace_adj<true, S><<<grid, 128, grad_smem(ab), st>>>(lc, ab);
+    if (ab.occluders) {
+        const u32 nee_blocks = (lc.total_nee / (ab.same_samples ? ab.same_samples : 1u) + 127) / 128;
+        k_nee_adj<S><<<nee_blocks + (u32)g_sm_count * 4u, 128, grad_smem(ab), st>>>(lc, ab, nee_blocks);
+    }
+}
 void launch_trace_adj(const LaunchCtx &lc, const AdjBufs &ab, cudaStream_t st) {
     if (!lc.total_pixels)
         return;
-    const u32 grid = (lc.total_pixels + 127) / 128;
-    if (!ab.tr.def_cnt) {
-        k_trace_adj<false><<<grid, 128, grad_smem(ab), st>>>(lc, ab);
-        return;
-    }
-    k_trace_adj<true><<<grid, 128, grad_smem(ab), st>>>(lc, ab);
-    if (ab.occluders) {
-        const u32 nee_blocks = (lc.total_nee / (ab.same_samples ? ab.same_samples : 1u) + 127) / 128;
-        k_nee_adj<<<nee_blocks + (u32)g_sm_count * 4u, 128, grad_smem(ab), st>>>(lc, ab, nee_blocks);
-    }
+    if (ab.block_sums)
+        launch_trace_adj_s<float>(lc, ab, st);
+    else
+        launch_trace_adj_s<double>(lc, ab, st);
 }
 void launch_emit_adj(const LaunchCtx &lc, const AdjBufs &ab, cudaStream_t st) {
     if (!lc.total_emit)
         return;
     cudaMemsetAsync(ab.n_paths, 0, sizeof(u32), st);
     k_adj_paths<<<(lc.total_emit + 255) / 256, 256, 0, st>>>(lc, ab);
-    k_emit_adj<<<(lc.total_emit + 127) / 128, 128, grad_smem(ab), st>>>(lc, ab);
+    const u32 grid = (lc.total_emit + 127) / 128;
+    if (ab.block_sums)
+        k_emit_adj<float><<<grid, 128, grad_smem(ab), st>>>(lc, ab);
+    else
+        k_emit_adj<double><<<grid, 128, 0, st>>>(lc, ab);
 }
 void launch_gather_adj(const LaunchCtx &lc, const GatherBufs &g, const AdjBufs &ab, cudaStream_t st) {
     if (lc.total_pixels)

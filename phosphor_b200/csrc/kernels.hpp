@@ -190,7 +190,7 @@ struct AdjBufs {
     TraceOut tr;           // the round's camera pass with its recorded NEE samples (def_cnt null: not recorded)
     u32 same_samples;      // direct_samples where a hit point's samples are all one ray, else 0
     u32 occluders;         // 1: materials transmit, the recorded samples' occluders are looked up
-    u32 block_sums;        // 1: per-block partial sums in 4*n_params bytes of shared memory
+    u32 block_sums;        // 1: per-block partial sums in 4*n_params bytes of shared memory; 0: all in double
 };
 void launch_gather_adj(const LaunchCtx &lc, const GatherBufs &g, const AdjBufs &ab, cudaStream_t st);
 void launch_trace_adj(const LaunchCtx &lc, const AdjBufs &ab, cudaStream_t st);

@@ -379,8 +379,9 @@ typedef struct phx_tuning {
                                    camera and photon passes on branches of their own (they depend only
                                    on the round seed) and the gathers in round order, so rounds overlap;
                                    up to k - 1 extra sets of per-round buffers (1..8, 1 = off; default 4
-                                   where three extra sets take at most 4 GB, else 2; fewer rounds are
-                                   captured where their sets do not fit) */
+                                   where three extra sets take at most 4 GB, else 2).  Where the sets do
+                                   not fit, two rounds are captured at a time, else one, until the
+                                   tuning is set again; a call that needs the sets' memory takes it */
     uint32_t gather_coop;       /* 1 = a warp stages each cell's photon records in shared memory and its
                                    lanes that need the cell walk them; 0 = one thread per pixel */
     uint32_t reserved[1];
@@ -468,6 +469,10 @@ PHX_API int phx_adjoint_backward(void *ctx, const float *dl_dimage, float *grad,
  * PHX_E_TIMEOUT with the flag in *err_flags.  No reference counterpart (the reference has no
  * device-side waits). */
 PHX_API int phx_selftest_lookback_timeout(int device, uint32_t n, uint32_t *err_flags);
+/* From here on the contexts used on the calling thread allocate at most `bytes` of device memory for their
+ * buffers (trees aside) and meet a full device after that; 0 lifts the limit.  What was left of the limit
+ * before goes to *left (0: there was none; may be NULL). */
+PHX_API int phx_selftest_device_limit(uint64_t bytes, uint64_t *left);
 
 /* ---- allocation-free exclusive scan -------------------------------------------------------------
  * No counterpart in the reference.  out[i] = in[0] + ... + in[i-1] over n uint32 elements (sums

@@ -445,6 +445,7 @@ PHX_API int phx_set_tuning(void *ctx, const phx_tuning *in) {
             return fail(PHX_E_INVALID, "pipeline_rounds must be at most 8");
         Engine *e = eng(ctx);
         e->tune = *in;
+        e->pipe_fits = Engine::MAX_PIPE;
         e->invalidate_graph(); // the next replay is captured with the new launch shape
         return PHX_OK;
     });
@@ -488,6 +489,15 @@ PHX_API int phx_selftest_lookback_timeout(int device, uint32_t n, uint32_t *err_
             return fail(PHX_E_CUDA, "self-test kernel failed");
         if (*err_flags & ERR_LOOKBACK_TIMEOUT)
             return fail(PHX_E_TIMEOUT, "look-back wait gave up as intended (tile 0 withheld)");
+        return PHX_OK;
+    });
+}
+
+PHX_API int phx_selftest_device_limit(uint64_t bytes, uint64_t *left) {
+    return guard([&]() -> int {
+        const uint64_t was = limit_device(bytes ? bytes : UINT64_MAX);
+        if (left)
+            *left = was == UINT64_MAX ? 0 : was;
         return PHX_OK;
     });
 }

@@ -28,20 +28,34 @@ int fail(int code, const std::string &msg) {
 
 void init_kernels(int device);
 
+// What this thread's buffers may still take (phx_selftest_device_limit); without a limit, everything.
+static thread_local uint64_t device_left = UINT64_MAX;
+
+uint64_t limit_device(uint64_t bytes) {
+    const uint64_t left = device_left;
+    device_left = bytes;
+    return left;
+}
+
 int DevBuf::alloc(size_t b) {
     release();
-    bytes = b;
-    if (cudaMalloc(&p, b ? b : 16) != cudaSuccess) {
+    if (b > device_left || cudaMalloc(&p, b ? b : 16) != cudaSuccess) {
         cudaGetLastError();
         p = nullptr;
         return fail(PHX_E_OOM, "device allocation of " + std::to_string(b) + " bytes failed");
     }
+    bytes = b;
+    if (device_left != UINT64_MAX)
+        device_left -= b;
     return PHX_OK;
 }
 
 void DevBuf::release() {
-    if (p && !view)
+    if (p && !view) {
         cudaFree(p);
+        if (device_left != UINT64_MAX)
+            device_left += bytes;
+    }
     p = nullptr;
     bytes = 0;
     view = false;
@@ -1173,6 +1187,28 @@ int Engine::alloc_round_sets(uint32_t sets, size_t *only_bytes) {
     return PHX_OK;
 }
 
+// Gives the extra sets beyond `keep` back, with every graph that uses one.
+void Engine::drop_round_sets(uint32_t keep) {
+    invalidate_graph();
+    for (; xsets.size() > keep; xsets.pop_back()) {
+        xbufs.back().release();
+        xbufs.pop_back();
+    }
+}
+
+// A buffer of at least `bytes`, for which the rounds in flight give their sets back if they must: they only
+// save time, and the next graph call takes them again if they fit.
+int Engine::ensure(DevBuf &b, size_t bytes) {
+    if (b.p && b.bytes >= bytes)
+        return PHX_OK;
+    int r = b.alloc(bytes);
+    if (r == PHX_E_OOM && !xsets.empty()) {
+        drop_round_sets(0);
+        r = b.alloc(bytes);
+    }
+    return r;
+}
+
 // Captures k rounds.  Round i (0..k-1) uses buffer set k-1-i, so the last round leaves its results
 // in the engine's own buffers (read-back and every other form see the latest round).  The seed
 // steps stay in order on the engine's stream (they advance one RNG state); each round's passes
@@ -1236,7 +1272,12 @@ int Engine::capture_pipelined(uint32_t k) {
         graph_pipe[k] = nullptr;
         return fail(PHX_E_CUDA, std::string("stream capture failed: ") + cudaGetErrorString(e));
     }
-    CK(cudaGraphInstantiate(&gexec_pipe[k], graph_pipe[k], 0));
+    e = cudaGraphInstantiate(&gexec_pipe[k], graph_pipe[k], 0);
+    if (e != cudaSuccess) {
+        gexec_pipe[k] = nullptr;
+        return fail(e == cudaErrorMemoryAllocation ? PHX_E_OOM : PHX_E_CUDA,
+                    std::string("graph instantiation failed: ") + cudaGetErrorString(e));
+    }
     return PHX_OK;
 }
 
@@ -1255,7 +1296,10 @@ int Engine::graph_rounds(uint32_t rounds) {
                 if (r != PHX_E_OOM)
                     return r;
                 cudaGetLastError();
-                pipe_fits = k - 1; // the sets of this many rounds do not fit beside the rest
+                // The sets of this many rounds do not fit: two rounds in flight, then one, and what their sets
+                // leave goes back, so that a nearly full device keeps the room that smaller groups leave it.
+                pipe_fits = k > 2 ? 2 : 1;
+                drop_round_sets(pipe_fits - 1);
                 continue;
             }
             CK(cudaGraphLaunch(gexec_pipe[k], st));
@@ -1759,9 +1803,7 @@ int Engine::image(uint32_t s, float exposure, int tonemap, uint64_t total_photon
     }
     const uint32_t n = S.desc.n_pixels;
     int r;
-    if (img_rgb.bytes < (size_t)n * 12 && (r = img_rgb.alloc((size_t)n * 12)))
-        return r;
-    if (img_ldr.bytes < (size_t)n * 3 && (r = img_ldr.alloc((size_t)n * 3)))
+    if ((r = ensure(img_rgb, (size_t)n * 12)) || (r = ensure(img_ldr, (size_t)n * 3)))
         return r;
     float inv_ph = total_photons > 0 ? 1.0f / (float)total_photons : 0.0f; // output.cpp:56-57
     float inv_r = rounds > 0 ? 1.0f / (float)rounds : 0.0f;

@@ -99,6 +99,7 @@ struct RoundSet {
     u32 *order = nullptr; // the gather's pixel order (set by the camera pass)
 };
 
+uint64_t limit_device(uint64_t bytes); // phx_selftest_device_limit; returns what was left before
 float ray_reach(float geom, const phx_light *l, uint32_t n);
 uint32_t light_sample_draws(const phx_light *l, uint32_t n, float total_lum);
 
@@ -173,6 +174,8 @@ class Engine {
     std::vector<SceneSlot> sc;
     uint32_t total_pixels = 0, total_emit = 0, total_cells = 0, total_nee = 0;
     uint64_t total_slots = 0, max_photons = 0;
+    static constexpr int MAX_PIPE = 8;
+    uint32_t pipe_fits = MAX_PIPE; // largest group whose buffer sets could be allocated under this tuning
     uint32_t key_bits = 1;
     phx_tuning tune{};
     int stage_state = 0;
@@ -195,6 +198,8 @@ class Engine {
     // their own, the gathers in round order; extra buffer sets for all but the last round
     uint32_t pipeline_rounds() const;
     int alloc_round_sets(uint32_t sets, size_t *only_bytes = nullptr);
+    void drop_round_sets(uint32_t keep);
+    int ensure(DevBuf &b, size_t bytes);
     int capture_pipelined(uint32_t k);
     bool halved_grids = false; // while capturing a group of three or more rounds
     uint32_t shared_blocks(uint32_t per_sm) const { return halved_grids ? (per_sm + 1) / 2 : per_sm; }
@@ -202,10 +207,8 @@ class Engine {
     std::vector<RoundSet> xsets;
     std::vector<cudaStream_t> pipe_st;
     std::vector<cudaEvent_t> pipe_ev;
-    static constexpr int MAX_PIPE = 8;
     cudaGraph_t graph_pipe[MAX_PIPE + 1] = {}; // by group size
     cudaGraphExec_t gexec_pipe[MAX_PIPE + 1] = {};
-    uint32_t pipe_fits = MAX_PIPE; // largest group whose buffer sets could be allocated
     int upload_scene(uint32_t i, const phx_scene &s, const phx_params &p, uint32_t *pix, uint32_t *emit,
                      uint32_t *cell, uint64_t *slot);
     int scene_photon_range(uint32_t s, uint32_t *off, uint32_t *n);

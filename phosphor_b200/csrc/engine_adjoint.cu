@@ -23,14 +23,6 @@ namespace phx {
             return fail(PHX_E_CUDA, std::string(#x) + ": " + cudaGetErrorString(e_));                                  \
     } while (0)
 
-namespace {
-int ensure(DevBuf &b, size_t bytes) {
-    if (b.p && b.bytes >= bytes)
-        return PHX_OK;
-    return b.alloc(bytes);
-}
-} // namespace
-
 uint32_t Engine::n_params() const {
     return sc.size() == 1 ? 4 * (uint32_t)sc[0].mats.size() + 3 * (uint32_t)sc[0].lights.size() : 0;
 }

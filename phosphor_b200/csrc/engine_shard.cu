@@ -191,8 +191,8 @@ int Engine::shard_nccl_init(const uint8_t *id) {
         return nccl_fail(api, nr, "ncclCommInitRank");
     nccl_comm = comm;
     int r;
-    if ((r = sh_pos.alloc(16 * max_photons)) || (r = sh_pd.alloc(8 * max_photons)) ||
-        (r = sh_cnt.alloc(4 * (size_t)shard.world)))
+    if ((r = ensure(sh_pos, 16 * max_photons)) || (r = ensure(sh_pd, 8 * max_photons)) ||
+        (r = ensure(sh_cnt, 4 * (size_t)shard.world)))
         return r;
     return PHX_OK;
 }

@@ -1376,8 +1376,12 @@ int Engine::autotune(uint32_t rounds, phx_tuning *chosen) {
     const size_t P = total_pixels, ns = sc.size();
     DevBuf keep;
     int r;
-    if ((r = keep.alloc(36 * P + 4 * ns)))
+    if ((r = ensure(keep, 36 * P + 4 * ns)))
         return r;
+    struct Release {
+        DevBuf &b;
+        ~Release() { b.release(); }
+    } release_keep{keep};
     char *k = keep.as<char>();
     CK(cudaMemcpy(k, flux.p, 16 * P, cudaMemcpyDeviceToDevice));
     CK(cudaMemcpy(k + 16 * P, radiance.p, 16 * P, cudaMemcpyDeviceToDevice));
@@ -1397,15 +1401,18 @@ int Engine::autotune(uint32_t rounds, phx_tuning *chosen) {
     CK(cudaEventCreate(&e0));
     CK(cudaEventCreate(&e1));
     // milliseconds per round of `rounds` graph-replayed rounds (rounded up to whole pipelined groups,
-    // after a warm-up that captures the graph)
+    // after a warm-up that captures the graph); PHX_E_OOM where groups of the tuning's size do not fit
     auto trial = [&](const phx_tuning &tt, float *ms) -> int {
         tune = tt;
+        pipe_fits = MAX_PIPE;
         invalidate_graph();
         const uint32_t k = pipeline_rounds();
         const uint32_t n = (rounds + k - 1) / k * k;
         int rr = graph_rounds(k); // capture + warm-up
         if (rr)
             return rr;
+        if (pipeline_rounds() != k)
+            return fail(PHX_E_OOM, "the rounds in flight do not fit in device memory");
         if (cudaEventRecord(e0, st) != cudaSuccess)
             return fail(PHX_E_CUDA, "event record failed");
         if ((rr = graph_rounds(n)))
@@ -1418,8 +1425,10 @@ int Engine::autotune(uint32_t rounds, phx_tuning *chosen) {
     };
     phx_tuning best = tune;
     float best_ms = 0.0f;
-    r = trial(best, &best_ms);
-    // coordinate descent over the knobs that leave every result bit-identical
+    while ((r = trial(best, &best_ms)) == PHX_E_OOM && pipe_fits < best.pipeline_rounds)
+        best.pipeline_rounds = pipe_fits; // the tuning's own rounds in flight do not fit
+    // coordinate descent over the knobs that leave every result bit-identical; a candidate whose groups do not
+    // fit in device memory is skipped
     auto knob = [&](uint32_t phx_tuning::*f, std::initializer_list<uint32_t> values) {
         for (uint32_t v : values) {
             if (r || best.*f == v)
@@ -1428,6 +1437,10 @@ int Engine::autotune(uint32_t rounds, phx_tuning *chosen) {
             c.*f = v;
             float ms = 0.0f;
             r = trial(c, &ms);
+            if (r == PHX_E_OOM) {
+                r = PHX_OK;
+                continue;
+            }
             if (!r && ms < best_ms) {
                 best_ms = ms;
                 best = c;
@@ -1443,28 +1456,11 @@ int Engine::autotune(uint32_t rounds, phx_tuning *chosen) {
     knob(&phx_tuning::concurrent_passes, {0u, 1u});
     knob(&phx_tuning::gather_sorted, {1u, 0u});
     knob(&phx_tuning::gather_coop, {1u, 0u});
-    // rounds in flight: each more needs another set of per-round buffers; a candidate whose sets do
-    // not fit in device memory is skipped
-    for (uint32_t v : {1u, 2u, 4u}) {
-        if (r || best.pipeline_rounds == v)
-            continue;
-        phx_tuning c = best;
-        c.pipeline_rounds = v;
-        float ms = 0.0f;
-        r = trial(c, &ms);
-        if (r == PHX_E_OOM) {
-            r = PHX_OK;
-            cudaGetLastError();
-            continue;
-        }
-        if (!r && ms < best_ms) {
-            best_ms = ms;
-            best = c;
-        }
-    }
+    knob(&phx_tuning::pipeline_rounds, {1u, 2u, 4u}); // each more needs another set of per-round buffers
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     tune = best;
+    pipe_fits = MAX_PIPE;
     invalidate_graph();
     // restore the state
     CK(cudaMemcpy(flux.p, k, 16 * P, cudaMemcpyDeviceToDevice));

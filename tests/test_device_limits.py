@@ -94,3 +94,20 @@ def test_later_calls_take_the_sets_memory():
     for a, b in zip(got, want):
         assert np.array_equal(a, b)
     assert np.abs(grad2 - grad).max() <= 1e-5 * np.abs(grad).max()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("start", [4, 2])
+@pytest.mark.parametrize("room,most", [(3.5, 4), (1.5, 2), (0.5, 1)])
+def test_autotune_keeps_to_groups_that_fit(start, room, most):
+    """The state that the tuner keeps aside (36 bytes a pixel) has its own room here."""
+    one = set_bytes()
+    with renderer() as r:
+        t = r.tuning()
+        t.pipeline_rounds = start
+        r.set_tuning(t)
+        with limit(int(room * one) + 40 * W * H) as taken:
+            chosen = r.autotune(4)
+            assert chosen.pipeline_rounds <= most
+            r.iterate(4)
+            assert taken() <= (most - 1) * one  # and the state kept aside is back

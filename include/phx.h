@@ -371,12 +371,12 @@ typedef struct phx_tuning {
     uint32_t emit_blocks_per_sm;
     uint32_t persistent;        /* 1 = persistent lane-refill kernels, 0 = one thread per item */
     uint32_t nee_wavefront;     /* 1 = diffuse-hit NEE shadow rays traced by a separate wavefront */
-    uint32_t concurrent_passes; /* 1 = a captured group of rounds (pipeline_rounds > 1) runs each round's
-                                   camera and photon passes on two branches (they only share the round
-                                   seed); rounds run one at a time always do */
+    uint32_t concurrent_passes; /* 1 = a captured group of three or more rounds runs each round's camera
+                                   and photon passes on two branches (they only share the round seed);
+                                   groups of two and rounds run one at a time always do */
     uint32_t gather_sorted;     /* 1 = the gather visits pixels grouped by photon-grid cell */
     uint32_t pipeline_rounds;   /* k > 1: graph replays capture up to k rounds at a time, each round's
-                                   camera and photon passes on branches of their own (they depend only
+                                   passes on a branch of their own (they depend only
                                    on the round seed) and the gathers in round order, so rounds overlap;
                                    up to k - 1 extra sets of per-round buffers (1..8, 1 = off; default 4
                                    where three extra sets take at most 4 GB, else 2).  Where the sets do
@@ -390,7 +390,8 @@ PHX_API int phx_get_tuning(void *ctx, phx_tuning *out);
 PHX_API int phx_set_tuning(void *ctx, const phx_tuning *in);
 /* Autotuner (no counterpart in the reference): times graph-replayed rounds of this context or batch
  * under candidate tunings — lane refill on/off, NEE wavefront on/off, persistent grid sizes of the
- * camera and photon kernels, concurrent passes on/off, 1/2/4 rounds in flight — by coordinate
+ * camera and photon kernels, 1/2/4 rounds in flight, concurrent passes on/off where that is a choice
+ * (three and more rounds in flight) — by coordinate
  * descent, keeps the fastest and writes it to *chosen (may be NULL).  Every candidate gives
  * bit-identical results; the SPPM state, seeds and round counters are restored afterwards.  Each
  * trial renders a warm-up group and rounds_per_trial rounds rounded up to whole groups

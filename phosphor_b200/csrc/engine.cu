@@ -1453,10 +1453,11 @@ int Engine::autotune(uint32_t rounds, phx_tuning *chosen) {
         knob(&phx_tuning::trace_blocks_per_sm, {2u, 4u, 6u, 8u, 12u, 16u});
         knob(&phx_tuning::emit_blocks_per_sm, {2u, 4u, 6u, 8u, 12u, 16u});
     }
-    knob(&phx_tuning::concurrent_passes, {0u, 1u});
     knob(&phx_tuning::gather_sorted, {1u, 0u});
     knob(&phx_tuning::gather_coop, {1u, 0u});
     knob(&phx_tuning::pipeline_rounds, {1u, 2u, 4u}); // each more needs another set of per-round buffers
+    if (best.pipeline_rounds > 2) // smaller groups are the same with and without
+        knob(&phx_tuning::concurrent_passes, {0u, 1u});
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     tune = best;

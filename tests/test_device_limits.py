@@ -111,3 +111,23 @@ def test_autotune_keeps_to_groups_that_fit(start, room, most):
             assert chosen.pipeline_rounds <= most
             r.iterate(4)
             assert taken() <= (most - 1) * one  # and the state kept aside is back
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("concurrent", [0, 1])
+def test_autotune_leaves_what_is_no_choice(concurrent):
+    """Groups of two are captured the same with and without concurrent_passes, so no trial times it."""
+    with renderer() as r:
+        t = r.tuning()
+        t.concurrent_passes = concurrent
+        r.set_tuning(t)
+        with limit(set_bytes_of(r) + 40 * W * H):
+            for _ in range(3):
+                chosen = r.autotune(2)
+                assert chosen.pipeline_rounds <= 2 and chosen.concurrent_passes == concurrent
+
+
+def set_bytes_of(r):
+    with limit(HUGE) as taken:
+        r.iterate(2)
+        return taken()

@@ -1237,10 +1237,10 @@ int Engine::capture_pipelined(uint32_t k) {
     // three and more rounds share the GPU better when each round's lane-refill kernels fill half of it (4 of 8
     // blocks per SM): 400 x 400 two lights 1.60 -> 1.50 ms a round, textured atrium 0.79 -> 0.75, sixteen small
     // scenes 1.27 -> 1.22, 512 x 512 Cornell 0.76 -> 0.74; two rounds do not (caustic 9.15 -> 9.38)
-    halved_grids = k >= 3;
     CK(cudaStreamSynchronize(st));
     CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
     capturing = true;
+    halved_grids = k >= 3;
     for (uint32_t i = 0; i < k; i++) {
         RoundSet &R = set(i);
         enq_seeds_r(R, st);

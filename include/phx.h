@@ -367,7 +367,8 @@ typedef struct phx_tuning {
     uint32_t trace_block;       /* threads per block, trace kernel */
     uint32_t emit_block;        /* threads per block, photon kernel */
     uint32_t gather_block;      /* threads per block, gather kernel */
-    uint32_t trace_blocks_per_sm;  /* persistent grid: resident blocks per SM */
+    uint32_t trace_blocks_per_sm;  /* persistent grid: resident blocks per SM (0: 8); half of it, rounded up,
+                                      in captured groups of three and more rounds, which share the GPU */
     uint32_t emit_blocks_per_sm;
     uint32_t persistent;        /* 1 = persistent lane-refill kernels, 0 = one thread per item */
     uint32_t nee_wavefront;     /* 1 = diffuse-hit NEE shadow rays traced by a separate wavefront */
@@ -474,6 +475,8 @@ PHX_API int phx_selftest_lookback_timeout(int device, uint32_t n, uint32_t *err_
  * buffers (trees aside) and meet a full device after that; 0 lifts the limit.  What was left of the limit
  * before goes to *left (0: there was none; may be NULL). */
 PHX_API int phx_selftest_device_limit(uint64_t bytes, uint64_t *left);
+/* Blocks per SM that a lane-refill kernel is launched with under a tuning's setting and rounds in flight. */
+PHX_API uint32_t phx_selftest_refill_blocks(uint32_t blocks_per_sm, uint32_t rounds_in_flight);
 
 /* ---- allocation-free exclusive scan -------------------------------------------------------------
  * No counterpart in the reference.  out[i] = in[0] + ... + in[i-1] over n uint32 elements (sums

@@ -502,6 +502,10 @@ PHX_API int phx_selftest_device_limit(uint64_t bytes, uint64_t *left) {
     });
 }
 
+PHX_API uint32_t phx_selftest_refill_blocks(uint32_t blocks_per_sm, uint32_t rounds_in_flight) {
+    return refill_blocks_per_sm(blocks_per_sm, rounds_in_flight);
+}
+
 PHX_API int phx_set_materials(void *ctx, const phx_material *materials, uint32_t n) {
     return guard([&]() -> int {
         return ctx ? eng(ctx)->set_materials(materials, n) : fail(PHX_E_INVALID, "null context");

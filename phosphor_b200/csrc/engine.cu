@@ -755,7 +755,7 @@ void Engine::enq_trace_r(RoundSet &R, cudaStream_t s) {
     const bool spec = spec_deferred();
     if (spec)
         cudaMemsetAsync(R.spec_next, 0, sizeof(u32), s);
-    launch_trace(l, o, (int)tune.trace_block, (int)tune.persistent, (int)shared_blocks(tune.trace_blocks_per_sm), R.queue,
+    launch_trace(l, o, (int)tune.trace_block, (int)tune.persistent, shared_blocks(tune.trace_blocks_per_sm), R.queue,
                  untextured(), s);
     ev(ST_TRACE, true, s);
     ev(ST_SHADOW, false, s);
@@ -791,7 +791,7 @@ void Engine::enq_emit_r(RoundSet &R, cudaStream_t s) {
     if (!in_adjoint)
         adj_live = ADJ_NO_ROUND;
     EmitOut o{R.slot_pos, R.slot_pd, R.counts, in_adjoint ? adj_slot_pow.as<float4>() : nullptr};
-    launch_emit(lc(R), o, (int)tune.emit_block, (int)tune.persistent, (int)shared_blocks(tune.emit_blocks_per_sm), R.queue + 1,
+    launch_emit(lc(R), o, (int)tune.emit_block, (int)tune.persistent, shared_blocks(tune.emit_blocks_per_sm), R.queue + 1,
                 untextured(), photon_prestart(), rough(), s);
     ev(ST_EMIT, true, s);
     ev(ST_EMIT_SCAN, false, s);
@@ -1234,13 +1234,10 @@ int Engine::capture_pipelined(uint32_t k) {
     // round 9.58 -> 9.45 ms, 1920 x 1080 atrium 5.88 -> 5.60, 333 x 251 0.69 -> 0.59); three and more fill the
     // GPU without (640 x 361 textured atrium 0.93 ms against 1.07 with)
     const bool branch = tune.concurrent_passes || k == 2;
-    // three and more rounds share the GPU better when each round's lane-refill kernels fill half of it (4 of 8
-    // blocks per SM): 400 x 400 two lights 1.60 -> 1.50 ms a round, textured atrium 0.79 -> 0.75, sixteen small
-    // scenes 1.27 -> 1.22, 512 x 512 Cornell 0.76 -> 0.74; two rounds do not (caustic 9.15 -> 9.38)
     CK(cudaStreamSynchronize(st));
     CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
     capturing = true;
-    halved_grids = k >= 3;
+    in_flight = k;
     for (uint32_t i = 0; i < k; i++) {
         RoundSet &R = set(i);
         enq_seeds_r(R, st);
@@ -1266,7 +1263,7 @@ int Engine::capture_pipelined(uint32_t k) {
     }
     perm = rs0.perm;
     capturing = false;
-    halved_grids = false;
+    in_flight = 1;
     cudaError_t e = cudaStreamEndCapture(st, &graph_pipe[k]);
     if (e != cudaSuccess) {
         graph_pipe[k] = nullptr;

@@ -201,8 +201,8 @@ class Engine {
     void drop_round_sets(uint32_t keep);
     int ensure(DevBuf &b, size_t bytes);
     int capture_pipelined(uint32_t k);
-    bool halved_grids = false; // while capturing a group of three or more rounds
-    uint32_t shared_blocks(uint32_t per_sm) const { return halved_grids ? (per_sm + 1) / 2 : per_sm; }
+    uint32_t in_flight = 1; // rounds of the group being captured
+    int shared_blocks(uint32_t per_sm) const { return (int)refill_blocks_per_sm(per_sm, in_flight); }
     std::vector<DevBuf> xbufs; // one per extra set
     std::vector<RoundSet> xsets;
     std::vector<cudaStream_t> pipe_st;

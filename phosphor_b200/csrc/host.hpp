@@ -29,6 +29,15 @@ struct PackedBvh {
 // Leaf rank of every triangle in the reference tree (pre-order over leaves): the tie-break key of
 // hits at exactly equal t (hit.h:68 keeps the last tested one).
 std::vector<uint32_t> reference_leaf_ranks(const std::vector<phx_bvh_node> &nodes, uint32_t n_tris);
+// Blocks per SM of a lane-refill kernel under the tuning's setting (0: the default, 8).  Three and more rounds
+// in flight share the GPU better when each fills half of it: 400 x 400 two lights 1.60 -> 1.50 ms a round,
+// textured atrium 0.79 -> 0.75, sixteen small scenes 1.27 -> 1.22, 512 x 512 Cornell 0.76 -> 0.74; two rounds
+// do not (caustic 9.15 -> 9.38).
+inline uint32_t refill_blocks_per_sm(uint32_t setting, uint32_t rounds_in_flight) {
+    const uint32_t n = setting ? setting : 8u;
+    return rounds_in_flight >= 3 ? (n + 1) / 2 : n;
+}
+
 // The reference tree itself re-packed as child pairs (one triangle per leaf).
 void bvh_pack(const std::vector<phx_bvh_node> &nodes, const phx_triangle *tris, PackedBvh &out);
 // A binned-SAH tree over the same expanded triangle boxes (bounding_box.h:48-61), leaves of up to

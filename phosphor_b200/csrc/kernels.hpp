@@ -214,11 +214,11 @@ void launch_next_seeds(u32 *state, u32 *seeds, u32 n, cudaStream_t st);
 
 // SM count of the current device (set by init_kernels, called once per engine outside capture)
 extern int g_sm_count;
-// Blocks of a lane-refill kernel (128 threads) over n items: per_sm (default 8) on every SM, but none that
+// Blocks of a lane-refill kernel (128 threads) over n items: per_sm on every SM, but none that
 // would find no item; the warps that only looked at the queue and left cost a 64 x 64 view's photon kernel
 // 0.137 ms against 0.110.
 inline int refill_grid(u32 n, int per_sm) {
-    const u32 most = (u32)g_sm_count * (u32)(per_sm > 0 ? per_sm : 8), need = n / 128u + (n % 128u != 0);
+    const u32 most = (u32)g_sm_count * (u32)per_sm, need = n / 128u + (n % 128u != 0);
     return (int)(need < most ? need : most);
 }
 void init_kernels(int device);

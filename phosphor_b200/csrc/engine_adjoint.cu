@@ -94,9 +94,12 @@ int Engine::adjoint_forward(uint32_t rounds, float *image) {
     const size_t rp = (size_t)rounds * P;
     int r;
     if ((r = ensure(adj_seeds, 4 * (size_t)rounds)) || (r = ensure(adj_r2, 4 * rp)) ||
-        (r = ensure(adj_ratio, 4 * rp)) || (r = ensure(adj_k, 4 * rp)) || (r = ensure(adj_img, 12 * (size_t)P)) ||
-        (r = ensure(adj_slot_pow, 16 * total_slots)))
+        (r = ensure(adj_ratio, 4 * rp)) || (r = ensure(adj_k, 4 * rp)) || (r = ensure(adj_img, 12 * (size_t)P)))
         return r;
+    // The photons' unquantised power (16 bytes a photon slot), which only the backward pass reads.  Where it
+    // does not fit, the forward pass goes without it and the backward pass renders the last round again.
+    const bool with_power = (adj_slot_pow.p && adj_slot_pow.bytes >= 16 * total_slots) ||
+                            adj_slot_pow.alloc(16 * total_slots) == PHX_OK;
     adj_ready = false;
     adj_live = ADJ_NO_ROUND;
     CK(cudaStreamSynchronize(st));
@@ -129,7 +132,8 @@ int Engine::adjoint_forward(uint32_t rounds, float *image) {
     adj_rounds = rounds;
     adj_ready = true;
     adj_k_ready = false;
-    adj_live = rounds - 1; // its hit points, samples and photons are in the buffers
+    if (with_power)
+        adj_live = rounds - 1; // its hit points, samples and photons are in the buffers
     return PHX_OK;
 }
 

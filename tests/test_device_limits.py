@@ -131,3 +131,26 @@ def set_bytes_of(r):
     with limit(HUGE) as taken:
         r.iterate(2)
         return taken()
+
+
+@pytest.mark.gpu
+def test_forward_pass_without_room_for_the_backward_pass():
+    """A forward pass needs no photon powers: it renders without them, the backward pass that finds no room
+    says so, and one that finds it gives the gradient."""
+    g = np.random.default_rng(1).standard_normal(W * H * 3).astype(np.float32)
+    with renderer() as r, limit(HUGE) as taken:
+        before = taken()
+        want = r.adjoint_forward(2).copy()
+        forward = taken() - before
+        grad = r.adjoint_backward(g)
+    slots = 16 * 4000 * 6  # photons per round, bounces
+    with renderer() as r:
+        with limit(forward - slots) as taken:
+            got = r.adjoint_forward(2)
+            assert np.array_equal(got.view(np.uint32), want.view(np.uint32))
+            assert taken() == forward - slots
+            with pytest.raises(A.PhxError) as e:
+                r.adjoint_backward(g)
+            assert e.value.code == A.PHX_E_OOM
+        for _ in range(2):
+            assert np.abs(r.adjoint_backward(g) - grad).max() <= 1e-5 * np.abs(grad).max()

@@ -166,6 +166,12 @@ static float ms_since(std::chrono::steady_clock::time_point t0) {
     return std::chrono::duration<float, std::milli>(std::chrono::steady_clock::now() - t0).count();
 }
 
+static float twice_area(const phx_triangle &t) {
+    const float ax = t.v1.x - t.v0.x, ay = t.v1.y - t.v0.y, az = t.v1.z - t.v0.z;
+    const float bx = t.v2.x - t.v0.x, by = t.v2.y - t.v0.y, bz = t.v2.z - t.v0.z;
+    const float x = ay * bz - az * by, y = az * bx - ax * bz, z = ax * by - ay * bx;
+    return std::sqrt(x * x + y * y + z * z);
+}
 // Largest |coordinate| of anything a ray starts from that does not change after set-up: the triangles
 // (`reach` so far), the emissive triangles and the camera.
 static float largest(const phx_f4 &p, float m) {
@@ -269,12 +275,20 @@ int Engine::upload_scene(uint32_t i, const phx_scene &s, const phx_params &p, ui
     if (!s.materials || s.n_materials == 0)
         return fail(PHX_E_INVALID, "scene has no materials");
     float reach = 0.0f;
+    std::vector<double> area(s.n_materials, 0.0);
     for (uint32_t t = 0; t < s.n_triangles; t++) {
         const phx_triangle &tr = s.triangles[t];
         if (tr.mat_index >= s.n_materials)
             return fail(PHX_E_INVALID, "triangle material index out of range");
         reach = largest(tr.v2, largest(tr.v1, largest(tr.v0, reach)));
+        area[tr.mat_index] += twice_area(tr);
     }
+    double all = 0.0;
+    for (double a : area)
+        all += a;
+    S.mat_area.resize(s.n_materials);
+    for (uint32_t m = 0; m < s.n_materials; m++)
+        S.mat_area[m] = (float)(area[m] / all);
     for (uint32_t l = 0; l < s.n_lights; l++)
         if (s.lights[l].kind == PHX_LIGHT_TEXTURED) {
             uint32_t a, b;
@@ -970,18 +984,19 @@ bool Engine::untextured() const {
     return true;
 }
 
-// Whether the mean over the scenes of their materials' mean roughness is 0.6 or more: between the
-// workloads that gain from searching the microfacet attempts (boxes with walls of roughness 1, with and
-// without glass: 0.71 and up; mixed batches: 0.7) and those that lose (atriums: 0.47).
+// Whether the roughness of the surfaces that a photon meets, by area and averaged over the scenes, is 0.7 or
+// more.  Photon kernel without and with the searched microfacet attempts, 2^18 photons, every surface of one
+// roughness: empty box 0.224 and 0.226 ms at 0.5, 0.229 and 0.228 at 0.6, 0.237 and 0.231 at 0.7, 0.274 and
+// 0.246 at 1; box with glass 0.816 and 0.832 at 0.6, 0.806 and 0.812 at 0.7, 0.802 and 0.798 at 0.8, 0.798
+// and 0.778 at 1; atrium, whose short paths seldom meet a warp's others, 3 to 7 % slower at any.  Mixed batches
+// of the three (0.75 to 0.83) gain 4 %, the atriums themselves (0.38 to 0.54) keep the kernel that is theirs.
 bool Engine::rough() const {
     double sum = 0.0;
-    for (const auto &s : sc) {
-        double m = 0.0;
-        for (const auto &mat : s.mats)
-            m += mat.roughness;
-        sum += m / (double)s.mats.size();
-    }
-    return sum >= 0.6 * (double)sc.size();
+    for (const auto &s : sc)
+        for (size_t m = 0; m < s.mats.size(); m++)
+            if (s.mat_area[m] > 0.0f)
+                sum += (double)s.mat_area[m] * s.mats[m].roughness;
+    return sum >= 0.7 * (double)sc.size();
 }
 
 bool Engine::photon_prestart() const {

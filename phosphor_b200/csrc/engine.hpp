@@ -37,6 +37,7 @@ struct SceneSlot {
     uint32_t trav_depth = 0, trav_inner = 0; // the device traversal tree
     float setup_ms = 0.0f, bvh_ms = 0.0f;     // wall time of the scene setup, of which the trees
     uint32_t n_tris = 0;
+    std::vector<float> mat_area; // share of the triangles' area that each material covers
     float geom_reach = 0.0f;  // largest |coordinate| of the triangles, camera and emissive triangles
     float box_reach = 0.0f;   // bound on every ray origin that the tree's boxes are made for (0: any)
     std::vector<DevBuf> bufs;

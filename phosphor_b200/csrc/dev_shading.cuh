@@ -229,10 +229,9 @@ PHX_DI float fma3(float a, float x, float b, float y, float c, float z) {
 }
 PHX_DI bool near_unit(float4 v) { return fabsf(fma3(v.x, v.x, v.y, v.y, v.z, v.z) - 1.0f) < 1e-5f; }
 
-// SEARCH: attempts are searched with a cheap test first (see below).
 // ggx_sample_vndf with the frame of `normal` (make_tbn) given by the caller; *refl receives
 // reflect(-view, h) when the accepted attempt computed it (*has_refl), as it does unless every
-// attempt failed and h is the normal.
+// attempt failed and h is the normal.  SEARCH: attempts are searched with a cheap test first.
 template <bool SEARCH = false>
 PHX_DI float4 ggx_sample_vndf_tbn(Rng *rng, float4 normal, float4 t, float4 b, float4 gn, float4 view,
                                   float roughness, float4 *refl_out, bool *has_refl) {
@@ -244,53 +243,8 @@ PHX_DI float4 ggx_sample_vndf_tbn(Rng *rng, float4 normal, float4 t, float4 b, f
     float4 T1 = (len_sq > 0.0f) ? f4(-vh.y, vh.x, 0.0f, 0.0f) * (1.0f / sqrtf(len_sq)) : f4(1.0f, 0.0f, 0.0f, 0.0f);
     float4 T2 = cross(vh, T1);
     float s = 0.5f * (1.0f + vh.z);
-    if constexpr (SEARCH) {
-    // An attempt's reflection is below the surface when 2 (v.h)(g.h) < (v.g) |h|^2 for the stretched
-    // half vector h in the frame of the normal.  That costs no division and no root, and where it holds
-    // by more than 1e-4 |h|^2 it decides as the exact arithmetic would (both err by under 1e-5 for unit
-    // vectors, which is checked; others, and NaNs, are always computed exactly).  So a warp's lanes,
-    // which need one to eight attempts each, search for a candidate with it and come together for the
-    // three normalisations.  The rougher the surface, the more attempts fail: photon kernel 0.271 ->
-    // 0.243 ms in the 512 x 512 Cornell box (roughness 1), 0.981 -> 0.939 in sixteen small scenes, but 2.25
-    // -> 2.33 in the atrium (0.05 to 0.9), where the test is one more thing to do; the engine picks.
-    const float gx = dot(gn, t), gy = dot(gn, b), gz = dot(gn, normal);
-    const float cvg = fma3(vl.x, gx, vl.y, gy, vl.z, gz) - 1e-4f;
-    const bool units = near_unit(view) && near_unit(gn) && near_unit(normal);
-    for (u32 a = 0;;) {
-        float4 hs;
-        bool rejected = true;
-        while (rejected && a < GGX_SAMPLING_ATTEMPTS) {
-            a++;
-            float u1 = random_float(rng);
-            float u2 = random_float(rng);
-            float r = sqrtf(u1);
-            float phi = (2.0f * PI) * u2;
-            float sp, cp;
-            pm_sincosf(phi, &sp, &cp);
-            float t1 = r * cp;
-            float t2 = r * sp;
-            t2 = (1.0f - s) * sqrtf(fmaxf(0.0f, 1.0f - t1 * t1)) + s * t2;
-            float nz2 = fmaxf(0.0f, 1.0f - t1 * t1 - t2 * t2);
-            float4 nh = t1 * T1 + t2 * T2 + sqrtf(nz2) * vh;
-            hs = f4(alpha * nh.x, alpha * nh.y, fmaxf(0.0f, nh.z), 0.0f);
-            rejected = units && 2.0f * fma3(vl.x, hs.x, vl.y, hs.y, vl.z, hs.z) * fma3(gx, hs.x, gy, hs.y, gz, hs.z) <
-                                    cvg * fma3(hs.x, hs.x, hs.y, hs.y, hs.z, hs.z);
-        }
-        if (rejected)
-            return normal;
-        float4 nel = normalize(hs);
-        float4 ne = normalize(nel.x * t + nel.y * b + nel.z * normal);
-        float4 refl = reflect(-view, ne);
-        if (dot(refl, gn) >= 0.0f) {
-            *refl_out = refl;
-            *has_refl = true;
-            return ne;
-        }
-        if (a == GGX_SAMPLING_ATTEMPTS)
-            return normal;
-    }
-    } else {
-    for (u32 a = 0; a < GGX_SAMPLING_ATTEMPTS; a++) {
+    // one attempt's half vector in the frame of the normal, stretched and not yet normalised
+    auto attempt = [&]() {
         float u1 = random_float(rng);
         float u2 = random_float(rng);
         float r = sqrtf(u1);
@@ -302,23 +256,55 @@ PHX_DI float4 ggx_sample_vndf_tbn(Rng *rng, float4 normal, float4 t, float4 b, f
         t2 = (1.0f - s) * sqrtf(fmaxf(0.0f, 1.0f - t1 * t1)) + s * t2;
         float nz2 = fmaxf(0.0f, 1.0f - t1 * t1 - t2 * t2);
         float4 nh = t1 * T1 + t2 * T2 + sqrtf(nz2) * vh;
-        float4 nel = normalize(f4(alpha * nh.x, alpha * nh.y, fmaxf(0.0f, nh.z), 0.0f));
-        float4 ne = normalize(nel.x * t + nel.y * b + nel.z * normal);
-        float4 refl = reflect(-view, ne);
-        if (dot(refl, gn) >= 0.0f) {
-            *refl_out = refl;
-            *has_refl = true;
-            return ne;
+        return f4(alpha * nh.x, alpha * nh.y, fmaxf(0.0f, nh.z), 0.0f);
+    };
+    // whether its reflection leaves the surface
+    auto accepted = [&](float4 hs, float4 *ne) {
+        float4 nel = normalize(hs);
+        *ne = normalize(nel.x * t + nel.y * b + nel.z * normal);
+        float4 refl = reflect(-view, *ne);
+        if (!(dot(refl, gn) >= 0.0f))
+            return false;
+        *refl_out = refl;
+        *has_refl = true;
+        return true;
+    };
+    float4 ne;
+    if constexpr (SEARCH) {
+        // An attempt's reflection is below the surface when 2 (v.h)(g.h) < (v.g) |h|^2 for the stretched
+        // half vector h in the frame of the normal.  That costs no division and no root, and where it holds
+        // by more than 1e-4 |h|^2 it decides as the exact arithmetic would (both err by under 1e-5 for unit
+        // vectors, which is checked; others, and NaNs, are always computed exactly).  So a warp's lanes,
+        // which need one to eight attempts each, search for a candidate with it and come together for the
+        // three normalisations.  The rougher the surface, the more attempts fail: photon kernel 0.271 ->
+        // 0.243 ms in the 512 x 512 Cornell box (roughness 1), 0.981 -> 0.939 in sixteen small scenes, but 2.25
+        // -> 2.33 in the atrium (0.05 to 0.9), where the test is one more thing to do; the engine picks.
+        const float gx = dot(gn, t), gy = dot(gn, b), gz = dot(gn, normal);
+        const float cvg = fma3(vl.x, gx, vl.y, gy, vl.z, gz) - 1e-4f;
+        const bool units = near_unit(view) && near_unit(gn) && near_unit(normal);
+        for (u32 a = 0;;) {
+            float4 hs;
+            bool rejected = true;
+            while (rejected && a < GGX_SAMPLING_ATTEMPTS) {
+                a++;
+                hs = attempt();
+                rejected = units && 2.0f * fma3(vl.x, hs.x, vl.y, hs.y, vl.z, hs.z) *
+                                            fma3(gx, hs.x, gy, hs.y, gz, hs.z) <
+                                        cvg * fma3(hs.x, hs.x, hs.y, hs.y, hs.z, hs.z);
+            }
+            if (rejected)
+                return normal;
+            if (accepted(hs, &ne))
+                return ne;
+            if (a == GGX_SAMPLING_ATTEMPTS)
+                return normal;
         }
+    } else {
+        for (u32 a = 0; a < GGX_SAMPLING_ATTEMPTS; a++)
+            if (accepted(attempt(), &ne))
+                return ne;
+        return normal;
     }
-    return normal;
-    }
-}
-PHX_DI float4 ggx_sample_vndf(Rng *rng, float4 normal, float4 gn, float4 view, float roughness) {
-    float4 t, b, refl;
-    bool has_refl;
-    make_tbn(normal, &t, &b);
-    return ggx_sample_vndf_tbn(rng, normal, t, b, gn, view, roughness, &refl, &has_refl);
 }
 
 PHX_DI float smith_g1_ggx(float c, float alpha) {

@@ -142,13 +142,8 @@ PHX_MATH_FN float pm_cosf(float x) {
 #define PM_LN2_HI 0.69140625f
 #define PM_LN2_LO 0.0017409306019544601f
 
-PHX_MATH_FN float pm_expf(float x) {
-    if (x != x)
-        return x;
-    if (x > 88.72283935546875f)
-        return pm_bits_to_f(0x7f800000u);
-    if (x < -103.97208404541016f)
-        return 0.0f;
+/* e^x 2^-k for the whole number k nearest to x / ln 2, |x| < 2^7 */
+PHX_MATH_FN float pm_exp_frac(float x, float *k) {
     float kf = floorf(x * PM_LOG2E + 0.5f);
     float r = x - kf * PM_LN2_HI;
     r = r - kf * PM_LN2_LO;
@@ -161,6 +156,18 @@ PHX_MATH_FN float pm_expf(float x) {
     p = p * r + 0.5f;
     p = p * r + 1.0f;
     p = p * r + 1.0f;
+    *k = kf;
+    return p;
+}
+
+PHX_MATH_FN float pm_expf(float x) {
+    if (x != x)
+        return x;
+    if (x > 88.72283935546875f)
+        return pm_bits_to_f(0x7f800000u);
+    if (x < -103.97208404541016f)
+        return 0.0f;
+    float kf, p = pm_exp_frac(x, &kf);
     int k = (int)kf;
     if (k < -126) {
         /* two-step scale keeps the intermediate normal */

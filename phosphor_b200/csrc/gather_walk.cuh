@@ -24,17 +24,8 @@ PHX_DI float div_gauss(float x) {
 
 // pm_expf for t in [-1, 0]: its operations without its range checks.
 PHX_DI float exp_unit(float t) {
-    const float kf = floorf(t * PM_LOG2E + 0.5f); // 0 or -1
-    float r = t - kf * PM_LN2_HI;
-    r = r - kf * PM_LN2_LO;
-    float p = 1.984126984126984e-04f;
-    p = p * r + 1.388888888888889e-03f;
-    p = p * r + 8.333333333333333e-03f;
-    p = p * r + 4.1666666666666664e-02f;
-    p = p * r + 1.6666666666666666e-01f;
-    p = p * r + 0.5f;
-    p = p * r + 1.0f;
-    p = p * r + 1.0f;
+    float kf; // 0 or -1
+    const float p = pm_exp_frac(t, &kf);
     return kf < 0.0f ? p * 0.5f : p;
 }
 

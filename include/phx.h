@@ -475,6 +475,10 @@ PHX_API int phx_selftest_lookback_timeout(int device, uint32_t n, uint32_t *err_
  * buffers (trees aside) and meet a full device after that; 0 lifts the limit.  What was left of the limit
  * before goes to *left (0: there was none; may be NULL). */
 PHX_API int phx_selftest_device_limit(uint64_t bytes, uint64_t *left);
+/* out[i] of one of the kernels' short forms, on the current device: 0 a byte over 255, 1 a[i] / b[i] with zero
+ * numerators apart, 2 a[i] / b[i] from the reciprocal, 3 a[i] over the gather kernel's denominator, 4 e^a[i] for
+ * a[i] in [-1, 0], 5 pm_expf(a[i]). */
+PHX_API int phx_selftest_math(int fn, const float *a, const float *b, float *out, uint32_t n);
 /* Blocks per SM that a lane-refill kernel is launched with under a tuning's setting and rounds in flight. */
 PHX_API uint32_t phx_selftest_refill_blocks(uint32_t blocks_per_sm, uint32_t rounds_in_flight);
 

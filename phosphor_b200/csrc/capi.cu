@@ -502,6 +502,15 @@ PHX_API int phx_selftest_device_limit(uint64_t bytes, uint64_t *left) {
     });
 }
 
+PHX_API int phx_selftest_math(int fn, const float *a, const float *b, float *out, uint32_t n) {
+    return guard([&]() -> int {
+        if (fn < 0 || fn > 5 || !a || !b || !out || n == 0 || n > (1u << 26))
+            return fail(PHX_E_INVALID, "bad arguments");
+        CK(selftest_math(fn, a, b, out, n));
+        return PHX_OK;
+    });
+}
+
 PHX_API uint32_t phx_selftest_refill_blocks(uint32_t blocks_per_sm, uint32_t rounds_in_flight) {
     return refill_blocks_per_sm(blocks_per_sm, rounds_in_flight);
 }

@@ -62,8 +62,9 @@ PHX_DI float4 srgb_to_linear(float4 c) {
     return f4(pm_powf(c.x, 2.2f), pm_powf(c.y, 2.2f), pm_powf(c.z, 2.2f), c.w);
 }
 
-// A byte over 255, rounded to nearest: one corrected step from the rounded reciprocal gives the quotient for
-// all 256 values (each was checked), in three instructions instead of a division.
+// A byte over 255, rounded to nearest: one of Markstein's correction steps (div_known, gather_walk.cuh) from the
+// rounded reciprocal gives the quotient for all 256 values (tests/test_short_forms.py), in three instructions
+// instead of a division.
 PHX_DI float unorm8(u8 b) {
     constexpr float r = 1.0f / 255.0f;
     const float x = (float)b, q = x * r;

@@ -15,7 +15,8 @@ PHX_DI float div_known(float x, float y, float r) {
     q = __fmaf_rn(__fmaf_rn(-q, y, x), r, q);
     return __fmaf_rn(__fmaf_rn(-q, y, x), r, q);
 }
-// x / GAUSS_DENOM for x = 0 or in [2^-30, 1.5]: one step is enough (every such x was checked).
+// x / GAUSS_DENOM for x = 0 or in [2^-30, 1.5]: one step is enough (tests/test_short_forms.py
+// tries every such x).
 PHX_DI float div_gauss(float x) {
     constexpr float r = 1.0f / GAUSS_DENOM;
     const float q = x * r;

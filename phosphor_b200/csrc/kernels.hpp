@@ -109,6 +109,7 @@ void launch_scan(const u32 *in, u32 *out, u64 n, void *scratch, u32 *total, u32 
                  const u32 *n_dyn = nullptr, u32 dyn_div = 1, u32 dyn_mul = 1);
 // failure-detection self-test: scan with tile 0 withheld; returns 0 ok, 2 alloc, 3 CUDA error
 int selftest_lookback_timeout(int device, u32 n, u32 *err_out);
+cudaError_t selftest_math(int fn, const float *a, const float *b, float *out, u32 n); // k_selftest.cu
 // exclusive scan with its scratch in a static device array (no allocation); synchronous.
 // returns 0 ok, 1 too large, 3 CUDA error, 4 look-back timeout (message in err)
 int scan_noalloc(const u32 *in, u32 *out, u32 n, u32 *total, cudaStream_t st, std::string &err);

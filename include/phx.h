@@ -276,7 +276,8 @@ PHX_API int phx_image(void *ctx, float exposure, int tonemap, uint64_t total_pho
 /* Bvh::Bvh (src/renderer/bvh.cpp:74-84): writes 2n-1 nodes; returns the tree depth in *depth. */
 PHX_API int phx_bvh_build(const phx_triangle *tris, uint32_t n, phx_bvh_node *out_nodes, uint32_t *depth);
 /* The traversal tree the kernels walk (no reference counterpart: the reference traverses the tree of
- * bvh.cpp): a binned-SAH tree over the reference's expanded triangle boxes with leaves of up to
+ * bvh.cpp): a binned-SAH tree over the reference's expanded triangle boxes (a context's own tree, but for
+ * PHX_F_QUANT_BVH, expands them by less where that holds every hit) with leaves of up to
  * max_leaf (1..16) triangles, as child pairs (wide = 0: 16 floats per inner node), collapsed to
  * 4-wide nodes (wide = 1: 28 floats) or 4-wide nodes with 8-bit child boxes (wide = 2: 16 words),
  * each triangle record (12 floats, leaf order) carrying its leaf rank in the
@@ -475,6 +476,10 @@ PHX_API int phx_selftest_lookback_timeout(int device, uint32_t n, uint32_t *err_
  * buffers (trees aside) and meet a full device after that; 0 lifts the limit.  What was left of the limit
  * before goes to *left (0: there was none; may be NULL). */
 PHX_API int phx_selftest_device_limit(uint64_t bytes, uint64_t *left);
+/* phx_traversal_bvh_build with the margin of a context whose rays start within `reach` of zero in each coordinate
+ * (0: the reference's margin). */
+PHX_API int phx_selftest_traversal_bvh(const phx_triangle *tris, uint32_t n, uint32_t max_leaf, int wide, int device,
+                                       float reach, phx_bvh_packed *out);
 /* out[i] of one of the kernels' short forms, on the current device: 0 a byte over 255, 1 a[i] / b[i] with zero
  * numerators apart, 2 a[i] / b[i] from the reciprocal, 3 a[i] over the gather kernel's denominator, 4 e^a[i] for
  * a[i] in [-1, 0], 5 pm_expf(a[i]). */

@@ -192,6 +192,8 @@ PROTOTYPES = [
     ("phx_stage_ms", C.c_int, [VP, C.POINTER(C.c_float), C.c_uint32]),
     ("phx_get_stream", C.c_uint64, [VP]),
     ("phx_selftest_device_limit", C.c_int, [C.c_uint64, C.POINTER(C.c_uint64)]),
+    ("phx_selftest_traversal_bvh", C.c_int, [C.POINTER(Triangle), C.c_uint32, C.c_uint32, C.c_int, C.c_int, C.c_float,
+                                             C.POINTER(BvhPacked)]),
     ("phx_selftest_math", C.c_int, [C.c_int, VP, VP, VP, C.c_uint32]),
     ("phx_selftest_refill_blocks", C.c_uint32, [C.c_uint32, C.c_uint32]),
     ("phx_selftest_lookback_timeout", C.c_int, [C.c_int, C.c_uint32, C.POINTER(C.c_uint32)]),

@@ -1,6 +1,7 @@
 // capi.cu — the extern "C" boundary of libphx.so (declared in include/phx.h).  Every entry point
 // validates its handle and arguments, catches every C++ exception and reports failures as status
 // codes with a message in phx_last_error(); nothing traps or throws across the boundary.
+#include "bvh_margin.hpp"
 #include "engine.hpp"
 #include "nccl_dl.hpp"
 
@@ -201,8 +202,9 @@ PHX_API int phx_bvh_build(const phx_triangle *tris, uint32_t n, phx_bvh_node *ou
     } while (0)
 #endif
 
-PHX_API int phx_traversal_bvh_build(const phx_triangle *tris, uint32_t n, uint32_t max_leaf, int wide, int device,
-                                    phx_bvh_packed *out) {
+// unit: the boxes' margin (bvh_margin.hpp), 0 for the reference's
+static int traversal_bvh(const phx_triangle *tris, uint32_t n, uint32_t max_leaf, int wide, int device, float unit,
+                         phx_bvh_packed *out) {
     return guard([&]() -> int {
         if (!tris || !out || !out->nodes || !out->trirec || !out->leaf_tri || n == 0 || max_leaf < 1 ||
             max_leaf > 16 || wide < 0 || wide > 2)
@@ -216,7 +218,7 @@ PHX_API int phx_traversal_bvh_build(const phx_triangle *tris, uint32_t n, uint32
         if (device < 0) {
             const auto t0 = std::chrono::steady_clock::now();
             PackedBvh pk;
-            if (!bvh_build_sah(tris, n, ranks, max_leaf, pk))
+            if (!bvh_build_sah(tris, n, ranks, max_leaf, pk, unit))
                 return fail(PHX_E_INVALID, "SAH build failed");
             if (wide)
                 bvh_widen(pk);
@@ -271,7 +273,7 @@ PHX_API int phx_traversal_bvh_build(const phx_triangle *tris, uint32_t n, uint32
         CK(cudaMemcpy(d_rank, ranks.data(), 4 * (size_t)n, cudaMemcpyHostToDevice));
         const auto t0 = std::chrono::steady_clock::now();
         std::string msg;
-        const int rc = bvh_device_build(d_tris, n, max_leaf, wide != 0, 0.0f, st, c.db, msg);
+        const int rc = bvh_device_build(d_tris, n, max_leaf, wide != 0, unit, st, c.db, msg);
         if (rc)
             return fail(rc == 2 ? PHX_E_OOM : rc == 1 ? PHX_E_INVALID : PHX_E_CUDA, msg);
         if (bvh_device_finish(d_tris, d_rank, n, c.db, d_rec, d_nrm, d_tan, d_uv, st))
@@ -291,6 +293,16 @@ PHX_API int phx_traversal_bvh_build(const phx_triangle *tris, uint32_t n, uint32
         CK(cudaMemcpy(out->leaf_tri, c.db.leaf_tri, 4 * (size_t)n, cudaMemcpyDeviceToHost));
         return PHX_OK;
     });
+}
+
+PHX_API int phx_traversal_bvh_build(const phx_triangle *tris, uint32_t n, uint32_t max_leaf, int wide, int device,
+                                    phx_bvh_packed *out) {
+    return traversal_bvh(tris, n, max_leaf, wide, device, 0.0f, out);
+}
+
+PHX_API int phx_selftest_traversal_bvh(const phx_triangle *tris, uint32_t n, uint32_t max_leaf, int wide, int device,
+                                       float reach, phx_bvh_packed *out) {
+    return traversal_bvh(tris, n, max_leaf, wide, device, tight_margin_unit(reach), out);
 }
 
 PHX_API int phx_hash_info(const phx_bvh_node *root, uint32_t grid_res, phx_photon_hash_data *out) {

@@ -623,9 +623,9 @@ int Engine::create(const phx_scene *scenes, const phx_params *params, uint32_t n
     tune.gather_sorted = 1;
     tune.gather_coop = 0; // the per-thread gather measured faster (caustic 2.28 vs 3.15 ms, atrium 3.52 vs 4.19)
     // Rounds in flight per graph replay: four where their three extra buffer sets take at most 4 GB, else
-    // two.  Smaller rounds leave more of the GPU idle: against two, 512 x 512 Cornell 0.84 -> 0.77 ms a
-    // round, 333 x 251 0.59 -> 0.50, sixteen small scenes 1.40 -> 1.26; the large workloads' sets take 3 to
-    // 10 GB each for 1 to 3 % (caustic 9.45 -> 9.2 ms, atrium 5.6 -> 5.4).
+    // two.  Smaller rounds leave more of the GPU idle: against two, 512 x 512 Cornell 0.82 -> 0.71 ms a
+    // round, 400 x 400 two lights 1.72 -> 1.48, sixteen small scenes 1.18 -> 1.01; the large workloads' sets
+    // take 3 to 10 GB each for 3 to 6 % (caustic 8.8 -> 8.5 ms, atrium 5.7 -> 5.4).
     size_t set_bytes = 0;
     alloc_round_sets(0, &set_bytes);
     tune.pipeline_rounds = 3 * set_bytes <= (4ull << 30) ? 4 : 2;

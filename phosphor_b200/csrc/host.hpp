@@ -30,9 +30,11 @@ struct PackedBvh {
 // hits at exactly equal t (hit.h:68 keeps the last tested one).
 std::vector<uint32_t> reference_leaf_ranks(const std::vector<phx_bvh_node> &nodes, uint32_t n_tris);
 // Blocks per SM of a lane-refill kernel under the tuning's setting (0: the default, 8).  Three and more rounds
-// in flight share the GPU better when each fills half of it: 400 x 400 two lights 1.60 -> 1.50 ms a round,
-// textured atrium 0.79 -> 0.75, sixteen small scenes 1.27 -> 1.22, 512 x 512 Cornell 0.76 -> 0.74; two rounds
-// do not (caustic 9.15 -> 9.38).
+// in flight share the GPU better when each fills half of it.  With four, milliseconds a round of full and half
+// grids: 400 x 400 two lights 1.59 and 1.48, textured atrium 0.78 and 0.73, sixteen small scenes 1.09 and 1.01,
+// 512 x 512 Cornell 0.74 and 0.71, caustic 8.54 and 8.54.  With three the small ones are even or gain
+// (0.76 and 0.73 Cornell, 1.13 and 1.15 sixteen scenes); the large ones, which get three only where a
+// caller asks for them, lose (caustic 8.6 and 9.0).  Two rounds do not gain (caustic 9.15 and 9.38).
 inline uint32_t refill_blocks_per_sm(uint32_t setting, uint32_t rounds_in_flight) {
     const uint32_t n = setting ? setting : 8u;
     return rounds_in_flight >= 3 ? (n + 1) / 2 : n;

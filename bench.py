@@ -719,7 +719,7 @@ def main() -> int:
     ap.add_argument("--pipeline-rounds", type=int, default=None,
                     help="rounds each graph replay captures and overlaps (1 = off; default: the library's)")
     ap.add_argument("--concurrent-passes", action="store_true",
-                    help="camera and photon passes on two branches of the captured round")
+                    help="camera and photon passes on two branches in captured groups of three and more rounds")
     ap.add_argument("--scale", type=int, default=1,
                     help="divide the resolution by s and the photon count by s^2 (small profiling cases only)")
     a = ap.parse_args()

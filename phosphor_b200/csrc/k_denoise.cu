@@ -209,7 +209,13 @@ static void fault_in(void *p, size_t bytes) {
     constexpr size_t PAGE = 4096, SHARE = (size_t)4 << 20;
     const size_t n = std::min<size_t>(std::min(8u, std::max(1u, std::thread::hardware_concurrency())), bytes / SHARE);
     cudaPointerAttributes at;
-    if (n < 2 || cudaPointerGetAttributes(&at, p) != cudaSuccess || at.type != cudaMemoryTypeUnregistered)
+    if (n < 2)
+        return;
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+        cudaGetLastError(); // not left for a later call to find
+        return;
+    }
+    if (at.type != cudaMemoryTypeUnregistered)
         return;
     std::vector<std::thread> threads;
     const size_t share = (bytes / n + PAGE - 1) / PAGE * PAGE;
